@@ -50,20 +50,18 @@ __device__ __forceinline__ Xyzz<F> negate(const Xyzz<F>& p) {
   return Xyzz<F>{p.x, neg(p.y), p.zz, p.zzz};
 }
 
-// 2P (dbl-2008-s-1, a = 0). Infinity stays infinity (ZZ = 0 gives ZZ3 = 0). The nine
-// products go in five steps of independent pairs.
+// 2P (dbl-2008-s-1, a = 0). Infinity stays infinity (ZZ = 0 gives ZZ3 = 0). Independent products
+// go in pairs; Y3 takes one reduction for its two products.
 template <class F>
 __device__ __forceinline__ Xyzz<F> xyzz_double(const Xyzz<F>& p) {
   F u = dbl(p.y);
-  F v, x2, w, s, m2, wy, zz3, zzz3;
+  F v, x2, w, s, zz3, zzz3;
   sqr2(u, p.x, v, x2);
   mul2(u, v, p.x, v, w, s);
   F m = dbl(x2) + x2;
-  mul2(m, m, w, p.y, m2, wy);
-  F x3 = m2 - dbl(s);
+  F x3 = sqr(m) - dbl(s);
   mul2(v, p.zz, w, p.zzz, zz3, zzz3);
-  F y3 = m * (s - x3) - wy;
-  return Xyzz<F>{x3, y3, zz3, zzz3};
+  return Xyzz<F>{x3, mul_sub(m, s - x3, w, p.y), zz3, zzz3};
 }
 
 // The doubling branch of the additions (P = Q) is rare; keeping it out of line keeps the hot
@@ -73,7 +71,8 @@ __device__ __noinline__ Xyzz<F> xyzz_double_call(Xyzz<F> p) {
   return xyzz_double(p);
 }
 
-// P + Q with Q affine (madd-2008-s): ten products in five pairs.
+// P + Q with Q affine (madd-2008-s): six products, two squares and R (Q - X3) - Y PPP through one
+// reduction.
 template <class F>
 __device__ __forceinline__ Xyzz<F> xyzz_add_affine(const Xyzz<F>& p, const Affine<F>& q) {
   if (is_infinity(q)) return p;
@@ -86,16 +85,16 @@ __device__ __forceinline__ Xyzz<F> xyzz_add_affine(const Xyzz<F>& p, const Affin
     if (r.is_zero()) return xyzz_double_call(p);
     return xyzz_infinity<F>();
   }
-  F ppsq, rr, ppp, q_, zz3, zzz3, t, yppp;
+  F ppsq, rr, ppp, q_, zz3, zzz3;
   sqr2(pp, r, ppsq, rr);
   mul2(pp, ppsq, p.x, ppsq, ppp, q_);
   F x3 = (rr - ppp) - dbl(q_);
-  mul2(r, q_ - x3, p.y, ppp, t, yppp);
+  const F y3 = mul_sub(r, q_ - x3, p.y, ppp);
   mul2(p.zz, ppsq, p.zzz, ppp, zz3, zzz3);
-  return Xyzz<F>{x3, t - yppp, zz3, zzz3};
+  return Xyzz<F>{x3, y3, zz3, zzz3};
 }
 
-// P + Q, both XYZZ (add-2008-s): fourteen products in seven pairs.
+// P + Q, both XYZZ (add-2008-s): ten products, two squares and R (Q - X3) - S1 PPP.
 template <class F>
 __device__ __forceinline__ Xyzz<F> xyzz_add(const Xyzz<F>& p, const Xyzz<F>& q) {
   if (is_infinity(q)) return p;
@@ -109,14 +108,14 @@ __device__ __forceinline__ Xyzz<F> xyzz_add(const Xyzz<F>& p, const Xyzz<F>& q) 
     if (r.is_zero()) return xyzz_double_call(p);
     return xyzz_infinity<F>();
   }
-  F ppsq, rr, ppp, q_, zz12, zzz12, t, sppp, zz3, zzz3;
+  F ppsq, rr, ppp, q_, zz12, zzz12, zz3, zzz3;
   sqr2(pp, r, ppsq, rr);
   mul2(pp, ppsq, u1, ppsq, ppp, q_);
   mul2(p.zz, q.zz, p.zzz, q.zzz, zz12, zzz12);
   F x3 = (rr - ppp) - dbl(q_);
-  mul2(r, q_ - x3, s1, ppp, t, sppp);
+  const F y3 = mul_sub(r, q_ - x3, s1, ppp);
   mul2(zz12, ppsq, zzz12, ppp, zz3, zzz3);
-  return Xyzz<F>{x3, t - sppp, zz3, zzz3};
+  return Xyzz<F>{x3, y3, zz3, zzz3};
 }
 
 // ------------------------------------------------------------------ inversion (Fermat)

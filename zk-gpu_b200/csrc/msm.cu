@@ -74,7 +74,6 @@ MsmPlan::MsmPlan(zkg_ctx* c_, int group_, size_t n_, uint32_t c, uint32_t item_p
   if (group != ZKG_G1 && group != ZKG_G2) fail(ZKG_EINVAL, "group must be ZKG_G1 or ZKG_G2");
   if (n >= (size_t)kNegBit) fail(ZKG_EINVAL, "an MSM holds fewer than 2^31 points");
   item_points_req = item_points;
-  const size_t max_entries = (size_t)((255 + c - 1) / c) * n;
 
   use(ctx);
   if (group == ZKG_G2) {
@@ -82,11 +81,12 @@ MsmPlan::MsmPlan(zkg_ctx* c_, int group_, size_t n_, uint32_t c, uint32_t item_p
     set_scan_smem_limits();
   }
   glv = glv_default();
-  // G1: FP64 limbs. With the GLV split one product per call at every size (measured: 2^16 1.27
-  // against 1.28 ms for two per call, 2^20 5.48 / 5.58, 2^22 15.60 / 16.05); with the plain
-  // windows two per call below 2^26 (window, point) entries, one above (3.5% faster at 2^20-2^21
-  // points, equal at 2^22, 3.5% slower from 2^23).
-  acc_variant = group == ZKG_G1 ? ((glv || (double)max_entries >= (double)(1u << 26)) ? 4 : 3) : 2;
+  // The plan's own choice, form 4 for G1 and form 2 for G2: integer products with interleaved
+  // accumulators (field.cuh), inlined for G1 and two per out-of-line call for G2. Accumulation,
+  // ms: G1 2^16 / 2^20 / 2^22 0.30 / 2.80 / 9.72, against 0.32 / 2.96 / 10.28 for one product
+  // per call, 0.31 / 2.94 / 10.24 for two and 0.40 / 3.88 / 13.05 for double-precision limbs; G2
+  // 2^20 9.79, against 10.0 for one per call, 11.2 inlined and 17.3 for limbs.
+  acc_variant = group == ZKG_G1 ? 4 : 2;
   chunk = std::min(n, max_chunk());
   layout();
   result.alloc(xyzz_words(), "msm result");
@@ -347,7 +347,7 @@ void MsmPlan::stage(int which, const uint32_t* bases, const uint32_t* scalars, c
         else
           msm_accumulate_f64<f64::FqD, true, true><<<grid_for(heads_max, 128), 128, acc_smem, s>>>(
               bases, bases2, split, sorted.ptr, slot_start.ptr, (uint32_t)active_slots(), seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
-      } else if (acc_variant >= 3) {
+      } else if (acc_variant == 3 || (acc_variant > 3 && std::is_same<F, Fq2>::value)) {
         using E = typename std::conditional<std::is_same<F, Fq>::value, f64::FqD, f64::Fq2D>::type;
         const size_t acc_smem = f64_acc_smem<E>();
         if (acc_variant == 3 || acc_variant == 6)

@@ -35,15 +35,12 @@ struct MsmPlan {
   int group;
   size_t n;
   uint32_t c, windows = 0, half = 0, seg_len = 0;
-  // Accumulation kernel form: 0 = field products inlined, 1 = through one out-of-line product
-  // (smaller code: the inlined mixed addition is thousands of instructions and its warps stall
-  // on instruction fetch; measured 17% faster at 2^24), 2 = out of line, independent products
-  // two per call, 3 / 4 = bucket arithmetic in double-precision limbs (msm_f64.cuh), two
-  // products per call / one. Every form fetches the next base into shared memory with
-  // cp.async. Defaults (measured on B200): G1 with the GLV split 4 at every size (2^20: 3.84
-  // against 3.95 ms for 3); G1 with the plain windows 3 below 2^26 (window, point) entries and 4
-  // above (2^24: 48.1 ms against 50.1 for 3 and 59.7 for 2; 2^20: 3.98 against 4.11 for 4), G2 2
-  // (47.4 ms at 2^22 against 48.1 for 1 and 55.9 / 63.0 for the limb forms 4 / 3). Tunable.
+  // Accumulation kernel form: 0 = integer field products inlined, 1 = through one out-of-line
+  // product, 2 = out of line, independent products two per call, 3 / 5 / 6 = bucket arithmetic in
+  // double-precision limbs (msm_f64.cuh: two products per call, or for G1 the accumulator in
+  // shared memory with one / two per call), 4 = for G1 the plan's own choice (inlined integer
+  // products), for G2 limbs with one product per call. Every form fetches the next base into
+  // shared memory with cp.async. Defaults (measured, MsmPlan's constructor): G1 4, G2 2. Tunable.
   int acc_variant = 4;
   // Warp aggregation of the counting pass's atomics (slot_peers in msm_kernels.cuh): 0 = every
   // group of equal slots, 1 = the first lane's group, 2 = none, 3 = the group of the first equal

@@ -59,8 +59,8 @@ std::vector<zkg_msm_tuning> tune_msm(zkg_ctx* ctx, int group, size_t n, const zk
           throw;
         }
         plan->check_buffers(bases, scalars);
-        // forms that can win: out-of-line integer products (1, 2) and, for G1, double-precision
-        // limbs (3, 4); fully inlined products (0) lose to both everywhere measured
+        // out-of-line integer products (1, 2) and, for G1, double-precision limbs (3) and the plan's
+        // own choice (4); form 0 is the same kernel as form 4 for G1 and loses to 1 and 2 for G2
         const std::vector<int> variants = group == ZKG_G1 ? std::vector<int>{1, 2, 3, 4} : std::vector<int>{1, 2};
         for (int v : variants) {
           plan->acc_variant = v;
