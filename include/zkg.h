@@ -277,12 +277,13 @@ int zkg_zkey_upload(zkg_ctx *ctx, const zkg_zkey *zkey, uint32_t section, zkg_bu
  * 9..=20, 16..256 points per accumulation thread, the accumulation kernel forms and, for G1 with
  * c <= 16, the GLV split on and off, and writes
  * up to cap results fastest first (out[0] is the choice; *count receives how many).
- * zkg_ntt_set_variant picks a plan's butterfly form: 0 = 32-bit integer products (tiles of 2^11
- * elements; default), 1 = double-precision limbs, products on the FP64 pipe (tiles of 2^10);
- * it resets the pass split to the form's default (at most 9 / 8 stages per pass).
- * zkg_ntt_set_max_stages picks the pass split (at most max_stages, 6..=11 for form 0, 6..=10
- * for form 1, stages per shared-memory pass); zkg_ntt_params reports form, split and passes.
- * zkg_tune_ntt times both forms and each split on `data` (forward + inverse, which leaves the
+ * zkg_ntt_set_variant picks a plan's butterfly form: 0 = 32-bit integer products, radix 2 (tiles of
+ * 2^11 elements), 1 = double-precision limbs, products on the FP64 pipe (tiles of 2^10), 2 = integer
+ * words, radix 4 in registers (default), 3 and 4 = double-precision limbs with staged twiddles, radix
+ * 2 and 4; it resets the pass split to the form's default (at most 9 stages per pass in form 0, 8 in
+ * the others). zkg_ntt_set_max_stages picks the pass split (at most max_stages, 6..=11 for form 0,
+ * 6..=10 for the others, stages per shared-memory pass); zkg_ntt_params reports form, split and passes.
+ * zkg_tune_ntt times every form and each split on `data` (forward + inverse, which leaves the
  * data unchanged) and returns the best. */
 typedef struct {
   uint32_t c, item_points;

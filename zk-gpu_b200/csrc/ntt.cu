@@ -5,12 +5,14 @@
 // Montgomery factor, so a Montgomery product x * tw returns exactly x * w^j (the reference's
 // convention, src/ntt.rs:3-5).
 //
-// The log_n stages run as passes over shared-memory tiles of 2^11 elements (64 KiB; three
-// tiles per SM): a pass of s stages loads 2^(11-s) consecutive columns of 2^s rows (rows are
-// 2^lm elements apart), so every global access is a run of at least four 32-byte elements.
+// The log_n stages run as passes over shared-memory tiles (2^11 elements in the radix-2 integer
+// form, at most 2^10 in the others): a pass of s stages on tiles of 2^tl elements loads 2^(tl-s)
+// consecutive columns of 2^s rows (rows are 2^lm elements apart), so global accesses are runs of
+// that many 32-byte elements.
 // The first pass reads the caller's buffer into the plan's scratch, middle passes work in
 // place on the scratch, and the last pass writes back in bit-reversed order (fused with the
-// 1/n scaling for the inverse). Transforms of at most 2^11 elements are one tile in one block.
+// 1/n scaling for the inverse). Transforms of at most one tile run in one block.
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <cstring>
@@ -261,6 +263,12 @@ __device__ __forceinline__ Fr quotient_element(const Fr& a, const Fr& b, const F
   return (a * b - c * one) * zinv2;
 }
 
+}  // namespace zkg
+
+#include "ntt_words.cuh"
+
+namespace zkg {
+
 // ------------------------------------------------------------------ staged-twiddle form
 //
 // The double-precision butterflies with each stage's twiddles copied into shared memory by
@@ -372,11 +380,12 @@ __device__ __forceinline__ void store_tile_f64(uint32_t* __restrict__ dst, const
   }
 }
 
-// One pass as ntt_pass_f64, with staged twiddles (tw: this pass's table, tw_mask = D - 1).
+// One pass as ntt_pass_f64, with staged twiddles (tw: this pass's table, tw_mask = D - 1), two
+// butterflies per thread step.
 // Shared memory: the tile (5 * elems doubles) and two twiddle buffers (stage 0, 2, ...: elems/2
 // entries; stage 1, 3, ...: elems/4), 70 KiB for tiles of 2^10 elements.
-template <bool LAST, bool PAIR>
-__global__ void __launch_bounds__(kNttThreads, PAIR ? 2 : 3)
+template <bool LAST>
+__global__ void __launch_bounds__(kNttThreads, 2)
     ntt_pass_f64s(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, const double* __restrict__ tw,
                   uint32_t tw_mask, uint32_t log_n, uint32_t tl, uint32_t lm, uint32_t s, int scale_flag,
                   Fr scale_mont, const uint32_t* __restrict__ sh_hi, const uint32_t* __restrict__ sh_lo,
@@ -403,8 +412,7 @@ __global__ void __launch_bounds__(kNttThreads, PAIR ? 2 : 3)
     const uint32_t lh = s - 1 - st;
     const uint32_t size = elems >> (st + 1);  // = 2^(lh + lg)
     const double* twst = (st & 1) ? twbuf1 : twbuf0;
-    if (PAIR && half_elems % (2 * kNttThreads) == 0) {
-      // two butterflies per iteration, loads first: two independent products in flight
+    {  // two butterflies per iteration (tiles of 2^10), loads first: two independent products in flight
       for (uint32_t b0 = threadIdx.x; b0 < half_elems; b0 += 2 * kNttThreads) {
         uint32_t sa[2], sb[2];
         FqD x[2], y[2], w[2];
@@ -434,34 +442,6 @@ __global__ void __launch_bounds__(kNttThreads, PAIR ? 2 : 3)
         tile_store_d(tile_d, elems, sb[0], o0);
         tile_store_d(tile_d, elems, sb[1], o1);
       }
-    } else
-    for (uint32_t b = threadIdx.x; b < half_elems; b += kNttThreads) {
-      const uint32_t col = b & ((1u << lg) - 1);
-      const uint32_t q = b >> lg;
-      const uint32_t r_lo = q & ((1u << lh) - 1);
-      const uint32_t row_a = ((q >> lh) << (lh + 1)) + r_lo;
-      const uint32_t slot_a = (row_a << lg) + col;
-      const uint32_t slot_b = slot_a + (1u << (lh + lg));
-      const uint32_t c = (tile << lg) + col;
-      const uint32_t j0 = c & ((1u << lm) - 1);
-      const FqD x = tile_load_d(tile_d, elems, slot_a);
-      const FqD y = tile_load_d(tile_d, elems, slot_b);
-      // Values enter even stages below 2r and odd stages below 4r: an even stage leaves its sums
-      // unreduced (below 4r) unless it is the pass's last; an odd stage reduces them (from below
-      // 8r). Differences get 4r added in odd stages, so products see inputs below 8r.
-      const bool odd = st & 1;
-      const FqD sum = fqd_add(x, y);
-      tile_store_d(tile_d, elems, slot_a, (odd || st + 1 == s) ? fqd_reduce<FrLimbs>(sum, kr) : sum);
-      const FqD d = odd ? fqd_sub<4, FrLimbs>(x, y) : fqd_sub<2, FrLimbs>(x, y);  // (0, 8r)
-      FqD out;
-      if ((r_lo | j0) != 0) {
-        const uint32_t e = b & (size - 1);
-        const FqD wd{{twst[e], twst[size + e], twst[2 * size + e], twst[3 * size + e], twst[4 * size + e]}};
-        out = fqd_mul<FrLimbs>(d, wd);
-      } else {
-        out = fqd_reduce<FrLimbs>(d, kr);
-      }
-      tile_store_d(tile_d, elems, slot_b, out);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
@@ -584,14 +564,10 @@ static void set_pass_smem_limits() {
              "ntt smem attribute");
   check_cuda(cudaFuncSetAttribute(ntt_pass<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
              "ntt smem attribute");
-  const int smem_s = (int)((size_t)70 << kTileLogD);  // tile + two twiddle buffers, forms 2 and 3
-  check_cuda(cudaFuncSetAttribute(ntt_pass_f64s<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_s),
+  const int smem_s = (int)((size_t)70 << kTileLogD);  // tile + two twiddle buffers, form 3
+  check_cuda(cudaFuncSetAttribute(ntt_pass_f64s<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_s),
              "ntt smem attribute");
-  check_cuda(cudaFuncSetAttribute(ntt_pass_f64s<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_s),
-             "ntt smem attribute");
-  check_cuda(cudaFuncSetAttribute(ntt_pass_f64s<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_s),
-             "ntt smem attribute");
-  check_cuda(cudaFuncSetAttribute(ntt_pass_f64s<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_s),
+  check_cuda(cudaFuncSetAttribute(ntt_pass_f64s<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_s),
              "ntt smem attribute");
   const int smem_r4 = (int)((size_t)80 << kTileLogD);  // tile + two step buffer sets, form 4
   check_cuda(cudaFuncSetAttribute(ntt_pass_f64r4<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_r4),
@@ -615,11 +591,10 @@ NttPlan::NttPlan(zkg_ctx* c, uint32_t log_n_) : ctx(c), log_n(log_n_) {
   build_seeds(w, seeds[0]);
   build_seeds(w_inv, seeds[1]);
   set_pass_smem_limits();
-  // Double-precision butterflies with staged twiddles by default, two per thread step up to 2^17
-  // elements: measured on B200 (ms per transform) 2^16: form 3 0.048, form 2 0.050, form 1
-  // 0.054, form 0 0.089; 2^20: form 2 0.292, form 3 0.302, form 1 0.313; 2^24: form 2 5.00,
-  // form 3 5.30, forms 0 and 1 5.33.
-  set_variant(log_n <= 17 ? 3 : 2);
+  // Integer words by default at every size. Measured on B200, us per forward transform, beside two
+  // double-precision butterflies per thread step (form 3): 2^12 20.5 / 39, 2^16 27.7 / 47, 2^20
+  // 195 / 300, 2^24 3230 / 5283.
+  set_variant(2);
 }
 
 uint32_t NttPlan::tile_log() const { return variant != 0 ? kTileLogD : kTileLog; }
@@ -667,8 +642,39 @@ bool NttPlan::set_max_stages(uint32_t ms) {
     passes.clear();
     for (uint32_t i = 0; i < p; i++) passes.push_back(log_n / p + (i < log_n % p ? 1u : 0u));
   }
-  if (variant >= 2) build_stage_tables();
+  if (variant == 2) build_words_tables();
+  else if (variant >= 3) build_stage_tables();
   return ok;
+}
+
+// The words form's tiles: 2^10 elements, fewer (down to one column) where the transform would
+// otherwise have less than 256 of them.
+void NttPlan::build_words_tables() {
+  use(ctx);
+  const uint32_t lo_bits = log_n / 2;  // as build_twiddles: ceil((log_n - 1) / 2)
+  for (int dir = 0; dir < 2; dir++) stage_tw[dir].clear();
+  stage_tw_mask.clear();
+  words_tile.clear();
+  uint32_t done = 0;
+  for (uint32_t st : passes) {
+    const uint32_t lm = log_n - done - st;
+    const uint32_t tl = std::max(st, std::min(kTileLogD, log_n > 8 ? log_n - 8 : 0u));
+    words_tile.push_back(tl);
+    const int spare = (int)log_n - (int)done - (int)tl;  // log2 of the distinct tile blocks
+    const size_t blocks = (size_t)1 << (spare > 0 ? spare : 0);
+    const size_t entries = blocks << tl;
+    stage_tw_mask.push_back((uint32_t)(blocks - 1));
+    for (int dir = 0; dir < 2; dir++) {
+      std::unique_ptr<DeviceArray> t(new DeviceArray);
+      t->alloc(8 * entries, "ntt pass twiddles");
+      ntt_words_twiddles<<<grid_for(entries, 256), 256, 0, ctx->setup>>>(seeds[dir][1].ptr, seeds[dir][0].ptr, lo_bits,
+                                                                         log_n, tl, lm, st, entries, t->ptr);
+      check_launch("ntt_words_twiddles");
+      stage_tw[dir].push_back(std::move(t));
+    }
+    done += st;
+  }
+  check_cuda(cudaStreamSynchronize(ctx->setup), "ntt pass twiddles");
 }
 
 void NttPlan::build_stage_tables() {
@@ -796,7 +802,11 @@ void NttPlan::enqueue(uint32_t* data, bool inverse, cudaStream_t s, const CosetS
     uint32_t* dst = last ? data : scratch.ptr;
     const int scale_flag = last && inverse;
     size_t ev = timer.enabled ? timer.begin((int)i, s) : 0;
-    const double* stw = variant >= 2 ? stage_tw[inverse ? 1 : 0][i]->as<double>() : nullptr;
+    const uint32_t* wtw = variant >= 2 ? stage_tw[inverse ? 1 : 0][i]->ptr : nullptr;
+    const double* stw = reinterpret_cast<const double*>(wtw);
+    const uint32_t wtl = variant == 2 ? words_tile[i] : 2;
+    const unsigned words_tiles = 1u << (log_n - wtl), words_threads = 1u << (wtl - 2);
+    const size_t words_smem = (size_t)32 << wtl;
     if (variant == 4 && last)
       ntt_pass_f64r4<true><<<tiles, kNttThreads, smem, s>>>(src, dst, stw, stage_tw_mask[i], log_n, tl, lm, st,
                                                             scale_flag, scale, sh_hi, sh_lo, sh_bits, qa, qb, qz2);
@@ -805,16 +815,18 @@ void NttPlan::enqueue(uint32_t* data, bool inverse, cudaStream_t s, const CosetS
                                                              scale_flag, scale, nullptr, nullptr, 0, nullptr, nullptr,
                                                              qz2);
     else if (variant == 2 && last)
-      ntt_pass_f64s<true, false><<<tiles, kNttThreads, smem, s>>>(src, dst, stw, stage_tw_mask[i], log_n, tl, lm,
-                                                                  st, scale_flag, scale, sh_hi, sh_lo, sh_bits, qa, qb, qz2);
+      ntt_pass_words<true><<<words_tiles, words_threads, words_smem, s>>>(src, dst, wtw, stage_tw_mask[i], log_n, words_tile[i],
+                                                               lm, st, scale_flag, scale, sh_hi, sh_lo, sh_bits, qa, qb,
+                                                               qz2);
     else if (variant == 2)
-      ntt_pass_f64s<false, false><<<tiles, kNttThreads, smem, s>>>(src, dst, stw, stage_tw_mask[i], log_n, tl, lm,
-                                                                   st, scale_flag, scale, nullptr, nullptr, 0, nullptr, nullptr, qz2);
+      ntt_pass_words<false><<<words_tiles, words_threads, words_smem, s>>>(src, dst, wtw, stage_tw_mask[i], log_n, words_tile[i],
+                                                                lm, st, scale_flag, scale, nullptr, nullptr, 0, nullptr,
+                                                                nullptr, qz2);
     else if (variant == 3 && last)
-      ntt_pass_f64s<true, true><<<tiles, kNttThreads, smem, s>>>(src, dst, stw, stage_tw_mask[i], log_n, tl, lm,
+      ntt_pass_f64s<true><<<tiles, kNttThreads, smem, s>>>(src, dst, stw, stage_tw_mask[i], log_n, tl, lm,
                                                                  st, scale_flag, scale, sh_hi, sh_lo, sh_bits, qa, qb, qz2);
     else if (variant == 3)
-      ntt_pass_f64s<false, true><<<tiles, kNttThreads, smem, s>>>(src, dst, stw, stage_tw_mask[i], log_n, tl, lm,
+      ntt_pass_f64s<false><<<tiles, kNttThreads, smem, s>>>(src, dst, stw, stage_tw_mask[i], log_n, tl, lm,
                                                                   st, scale_flag, scale, nullptr, nullptr, 0, nullptr,
                                                                   nullptr, qz2);
     else if (variant == 1 && last)

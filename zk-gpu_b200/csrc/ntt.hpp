@@ -32,11 +32,12 @@ struct NttPlan {
   StageTimer timer;  // one stage id per pass
 
   NttPlan(zkg_ctx* ctx, uint32_t log_n);
-  // Butterfly form: 0 = 32-bit integer products, 1 = double-precision limbs with twiddles read
-  // from a table of w^j, 2 = double-precision limbs with each stage's twiddles staged into shared
-  // memory from per-pass tables in butterfly order. Resets the pass split to the form's default.
-  // The first switch to form 1 builds its twiddle limbs; form 2 builds its tables for each split
-  // (set-up stream, waited for).
+  // Butterfly form: 0 = 32-bit integer products, radix 2 in shared memory, 1 = double-precision
+  // limbs with twiddles read from a table of w^j, 2 (default) = integer words, radix 4 in registers
+  // (ntt_words.cuh), 3 = double-precision limbs with each stage's twiddles staged into shared
+  // memory, 4 = the same in radix 4. Forms 2-4 read per-pass tables in butterfly order. Resets the
+  // pass split to the form's default. The first switch to form 1 builds its twiddle limbs; forms
+  // 2-4 build their tables for each split (set-up stream, waited for).
   bool set_variant(int variant);
   int variant = 2;
   uint32_t tile_log() const;
@@ -49,7 +50,7 @@ struct NttPlan {
   // (the same result as the transform followed by shift->enqueue, without another pass over
   // the data); the double-precision form runs the shift as its own kernel.
   // With `quot` (forward only), the output is (a b - NTT(data)) zinv instead (fused into the
-  // last pass in forms 2 and 3; the other forms run the quotient kernel after the transform).
+  // last pass in forms 2-4; the other forms run the quotient kernel after the transform).
   void enqueue(uint32_t* data, bool inverse, cudaStream_t s, const CosetShift* shift = nullptr,
                const Quotient* quot = nullptr);
   void run(zkg_buf* data, bool inverse, const CosetShift* shift = nullptr, const Quotient* quot = nullptr);
@@ -61,8 +62,10 @@ struct NttPlan {
  private:
   void build_seeds(const host::U256& root, DeviceArray (&seed)[2]);
   void build_twiddles(DeviceArray (&seed)[2], DeviceArray& out);
-  // Form 2: one table per pass and direction, for the split in `passes`.
+  // Forms 3 and 4, and form 2: one table per pass and direction, for the split in `passes`.
   void build_stage_tables();
+  void build_words_tables();
+  std::vector<uint32_t> words_tile;  // log2 of the tile, per pass
   std::vector<std::unique_ptr<DeviceArray>> stage_tw[2];
   std::vector<uint32_t> stage_tw_mask;  // tables' block count - 1, per pass
   struct FusedShift {

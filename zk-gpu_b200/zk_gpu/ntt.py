@@ -47,9 +47,9 @@ class Ntt:
         check(lib().zkg_ntt_forward_quotient(self._h, data.handle, a.handle, b.handle, _fr_words(g)))
 
     def set_variant(self, variant: int) -> None:
-        """Butterfly form: 0 = 32-bit integer products, 1 = double-precision limbs with twiddles
-        read from a table of powers, 2 = double-precision limbs with each stage's twiddles staged
-        into shared memory, 3 = form 2 with two butterflies per thread step."""
+        """Butterfly form: 0 = 32-bit integer products, radix 2, 1 = double-precision limbs with
+        twiddles read from a table of powers, 2 = integer words, radix 4 in registers (default),
+        3 / 4 = double-precision limbs with staged twiddles, radix 2 / 4."""
         check(lib().zkg_ntt_set_variant(self._h, variant))
 
     def set_max_stages(self, max_stages: int) -> None:
