@@ -592,8 +592,8 @@ NttPlan::NttPlan(zkg_ctx* c, uint32_t log_n_) : ctx(c), log_n(log_n_) {
   build_seeds(w_inv, seeds[1]);
   set_pass_smem_limits();
   // Integer words by default at every size. Measured on B200, us per forward transform, beside two
-  // double-precision butterflies per thread step (form 3): 2^12 20.5 / 39, 2^16 27.7 / 47, 2^20
-  // 195 / 300, 2^24 3230 / 5283.
+  // double-precision butterflies per thread step (form 3): 2^12 19.5 / 39, 2^16 24.7 / 47, 2^20
+  // 175 / 300, 2^24 2853 / 5283.
   set_variant(2);
 }
 
@@ -647,8 +647,11 @@ bool NttPlan::set_max_stages(uint32_t ms) {
   return ok;
 }
 
-// The words form's tiles: 2^10 elements, fewer (down to one column) where the transform would
-// otherwise have less than 256 of them.
+// The words form's tiles: 2^9 elements above 2^20 (runs of two columns: 64 bytes, what DRAM gives at
+// least), 2^8 up to there (the data stays in L2), fewer where the transform would otherwise have
+// less than 256 tiles; a pass of more stages takes tiles of one column. Smaller blocks spread an SM's
+// loads and stores between the others' products: us per forward transform with tiles of 2^8 / 2^9 /
+// 2^10 elements, 2^18 56 / 61 / 61, 2^20 175 / 178 / 188, 2^22 705 / 697 / 750, 2^24 3200 / 2853 / 3089.
 void NttPlan::build_words_tables() {
   use(ctx);
   const uint32_t lo_bits = log_n / 2;  // as build_twiddles: ceil((log_n - 1) / 2)
@@ -658,7 +661,7 @@ void NttPlan::build_words_tables() {
   uint32_t done = 0;
   for (uint32_t st : passes) {
     const uint32_t lm = log_n - done - st;
-    const uint32_t tl = std::max(st, std::min(kTileLogD, log_n > 8 ? log_n - 8 : 0u));
+    const uint32_t tl = std::max(st, std::min(log_n > 20 ? 9u : 8u, log_n > 8 ? log_n - 8 : 0u));
     words_tile.push_back(tl);
     const int spare = (int)log_n - (int)done - (int)tl;  // log2 of the distinct tile blocks
     const size_t blocks = (size_t)1 << (spare > 0 ? spare : 0);
@@ -666,7 +669,7 @@ void NttPlan::build_words_tables() {
     stage_tw_mask.push_back((uint32_t)(blocks - 1));
     for (int dir = 0; dir < 2; dir++) {
       std::unique_ptr<DeviceArray> t(new DeviceArray);
-      t->alloc(8 * entries, "ntt pass twiddles");
+      t->alloc(16 * entries, "ntt pass twiddles");
       ntt_words_twiddles<<<grid_for(entries, 256), 256, 0, ctx->setup>>>(seeds[dir][1].ptr, seeds[dir][0].ptr, lo_bits,
                                                                          log_n, tl, lm, st, entries, t->ptr);
       check_launch("ntt_words_twiddles");
@@ -814,14 +817,17 @@ void NttPlan::enqueue(uint32_t* data, bool inverse, cudaStream_t s, const CosetS
       ntt_pass_f64r4<false><<<tiles, kNttThreads, smem, s>>>(src, dst, stw, stage_tw_mask[i], log_n, tl, lm, st,
                                                              scale_flag, scale, nullptr, nullptr, 0, nullptr, nullptr,
                                                              qz2);
-    else if (variant == 2 && last)
-      ntt_pass_words<true><<<words_tiles, words_threads, words_smem, s>>>(src, dst, wtw, stage_tw_mask[i], log_n, words_tile[i],
-                                                               lm, st, scale_flag, scale, sh_hi, sh_lo, sh_bits, qa, qb,
-                                                               qz2);
-    else if (variant == 2)
-      ntt_pass_words<false><<<words_tiles, words_threads, words_smem, s>>>(src, dst, wtw, stage_tw_mask[i], log_n, words_tile[i],
-                                                                lm, st, scale_flag, scale, nullptr, nullptr, 0, nullptr,
-                                                                nullptr, qz2);
+    else if (variant == 2) {
+      auto launch = [&](auto kernel) {
+        kernel<<<words_tiles, words_threads, words_smem, s>>>(src, dst, wtw, stage_tw_mask[i], log_n, wtl, lm, st, scale_flag,
+                                                              scale, last ? sh_hi : nullptr, last ? sh_lo : nullptr,
+                                                              last ? sh_bits : 0, last ? qa : nullptr,
+                                                              last ? qb : nullptr, qz2);
+      };
+      if (words_threads > 128) launch(last ? ntt_pass_words<true, 256, 3> : ntt_pass_words<false, 256, 3>);
+      else if (words_threads > 64) launch(last ? ntt_pass_words<true, 128, 6> : ntt_pass_words<false, 128, 6>);
+      else launch(last ? ntt_pass_words<true, 64, 10> : ntt_pass_words<false, 64, 10>);
+    }
     else if (variant == 3 && last)
       ntt_pass_f64s<true><<<tiles, kNttThreads, smem, s>>>(src, dst, stw, stage_tw_mask[i], log_n, tl, lm,
                                                                  st, scale_flag, scale, sh_hi, sh_lo, sh_bits, qa, qb, qz2);

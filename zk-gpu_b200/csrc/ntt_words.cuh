@@ -1,19 +1,20 @@
-// NTT passes on 32-bit words: radix-4 butterflies in registers, integer Montgomery products
-// (field.cuh) with unreduced sums.
+// NTT passes on 32-bit words: radix-4 butterflies in registers, products by twiddles with a
+// precomputed quotient (field_shoup.cuh), unreduced sums.
 //
 // A pass of s stages works on tiles of 2^tl elements, 2^(tl - s) columns of 2^s rows. A thread
 // holds four rows of one column and runs two stages on them per step; between steps the tile goes
 // through shared memory (16-byte pieces, one array per half element, so that neighbouring lanes
 // never share a bank), the first step reads global memory and the last one writes it. What bounds
-// the pass is the wide multiply-add pipe: four products (528 of its slots) per four elements and
-// step beside ~480 add-pipe instructions; a butterfly takes about 260 instructions, where the
-// double-precision form of the same butterfly took about 570.
+// the pass is the wide multiply-add pipe: four products (428 of its slots) per four elements and
+// step beside ~400 add-pipe instructions; a butterfly takes about 240 instructions, where the
+// double-precision form of the same butterfly took about 570. At 2^22 the pipe is 60-76% busy in a
+// pass; the rest goes to the tiles' loads and stores, which other blocks' products cover in part.
 //
 // Bounds: r < 0.19 2^256, so 5r < 2^256. Elements between steps are below 2r; a sum of two is
-// brought below 2r again by one conditional subtraction of 2r, a difference gets 2r added and is a
-// product's operand (below 4r: product below 1.8r). Twiddles are reduced.
+// brought below 2r again by one conditional subtraction of 2r, and so is a product (below 2.8r); a
+// difference gets 2r added and is a product's operand (below 4r).
 #pragma once
-#include "field.cuh"
+#include "field_shoup.cuh"
 
 namespace zkg {
 namespace words {
@@ -105,8 +106,8 @@ __device__ __forceinline__ Rows rows_of(uint32_t u, uint32_t lg, uint32_t gap_lo
 
 }  // namespace words
 
-// The pass table for tiles of 2^tl elements (ntt_stage_twiddles' order, 32-byte Montgomery words per
-// entry): a block of 2^tl entries per distinct tile, stage st's 2^(tl - st - 1) twiddles from entry
+// The pass table for tiles of 2^tl elements (ntt_stage_twiddles' order, a shoup::Constant of 64 bytes
+// per entry): a block of 2^tl entries per distinct tile, stage st's 2^(tl - st - 1) twiddles from entry
 // 2^tl - 2^(tl - st) on, butterfly b's at b mod their number.
 __global__ void ntt_words_twiddles(const uint32_t* __restrict__ hi, const uint32_t* __restrict__ lo, uint32_t lo_bits,
                                    uint32_t log_n, uint32_t tl, uint32_t lm, uint32_t s, size_t entries,
@@ -121,15 +122,17 @@ __global__ void ntt_words_twiddles(const uint32_t* __restrict__ hi, const uint32
   const uint32_t e = off - (elems - (elems >> st));
   const uint32_t j0 = ((block << lg) + (e & ((1u << lg) - 1))) & ((1u << lm) - 1);
   const uint32_t idx = (((e >> lg) << lm) + j0) << (log_n - lm - s + st);  // < n / 2
-  store_fe(out + 8 * id, load_fe<Fr>(hi + 8 * (size_t)(idx >> lo_bits)) *
-                             load_fe<Fr>(lo + 8 * (size_t)(idx & ((1u << lo_bits) - 1))));
+  const shoup::Constant c = shoup::constant(load_fe<Fr>(hi + 8 * (size_t)(idx >> lo_bits)) *
+                                            load_fe<Fr>(lo + 8 * (size_t)(idx & ((1u << lo_bits) - 1))));
+  store_fe(out + 16 * id, c.w);
+  store_fe(out + 16 * id + 8, c.quotient);
 }
 
 // One pass: stages [log_n - lm - s, log_n - lm), 2 <= s <= tl, with 2^(tl - 2) threads. LAST writes
 // canonical words in natural order, with the 1/n scaling of an inverse, the fused coset shift
 // (sh_hi != null) or the fused quotient (qa != null).
-template <bool LAST>
-__global__ void __launch_bounds__(256, 3)
+template <bool LAST, uint32_t THREADS, uint32_t BLOCKS>
+__global__ void __launch_bounds__(THREADS, BLOCKS)
     ntt_pass_words(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, const uint32_t* __restrict__ tw,
                    uint32_t tw_mask, uint32_t log_n, uint32_t tl, uint32_t lm, uint32_t s, int scale_flag, Fr scale,
                    const uint32_t* __restrict__ sh_hi, const uint32_t* __restrict__ sh_lo, uint32_t sh_bits,
@@ -137,11 +140,13 @@ __global__ void __launch_bounds__(256, 3)
   using namespace words;
   extern __shared__ __align__(16) uint4 pieces[];  // low halves of the tile's elements, then high halves
   const uint32_t lg = tl - s, tile = blockIdx.x, elems = 1u << tl;
-  const uint32_t* const table = tw + 8 * ((size_t)(tile & tw_mask) << tl);
-  auto twiddle = [&](uint32_t st, uint32_t e) {
-    const uint4* p = reinterpret_cast<const uint4*>(table + 8 * (size_t)(elems - (elems >> st) + e));
-    const uint4 lo = __ldg(p), hi = __ldg(p + 1);
-    return Fr{{lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w}};
+  const uint32_t* const table = tw + 16 * ((size_t)(tile & tw_mask) << tl);
+  // x times twiddle e of stage st, below 2r
+  auto times = [&](const Fr& x, uint32_t st, uint32_t e) {
+    const uint4* p = reinterpret_cast<const uint4*>(table + 16 * (size_t)(elems - (elems >> st) + e));
+    const uint4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2), d = __ldg(p + 3);
+    return reduce_2r(shoup::mul(x, shoup::Constant{Fr{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}},
+                                                   Fr{{c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w}}}));
   };
   Fr v[4];
   for (uint32_t st = 0; st < s; st += 2) {
@@ -166,17 +171,16 @@ __global__ void __launch_bounds__(256, 3)
       const uint32_t e0 = ((at.row & (at.gap - 1)) << lg) + at.col;
       const Fr y0 = reduce_2r(add_raw(v[0], v[2])), y1 = reduce_2r(add_raw(v[1], v[3]));
       Fr y2 = sub_raw(v[0], v[2]);
-      y2 = unit ? reduce_2r(y2) : mont_mul_lazy(y2, twiddle(st, e0));
-      const Fr y3 = mont_mul_lazy(sub_raw(v[1], v[3]), twiddle(st, e0 + gap));
+      y2 = unit ? reduce_2r(y2) : times(y2, st, e0);
+      const Fr y3 = times(sub_raw(v[1], v[3]), st, e0 + gap);
       v[0] = reduce_2r(add_raw(y0, y1));
       v[2] = reduce_2r(add_raw(y2, y3));
       if (unit) {
         v[1] = reduce_2r(sub_raw(y0, y1));
         v[3] = reduce_2r(sub_raw(y2, y3));
       } else {
-        const Fr w = twiddle(st + 1, e0);
-        v[1] = mont_mul_lazy(sub_raw(y0, y1), w);
-        v[3] = mont_mul_lazy(sub_raw(y2, y3), w);
+        v[1] = times(sub_raw(y0, y1), st + 1, e0);
+        v[3] = times(sub_raw(y2, y3), st + 1, e0);
       }
     } else {  // rows (0, 1) and (2, 3)
       Fr d0 = sub_raw(v[0], v[1]), d1 = sub_raw(v[2], v[3]);
@@ -186,9 +190,8 @@ __global__ void __launch_bounds__(256, 3)
         v[1] = reduce_2r(d0);
         v[3] = reduce_2r(d1);
       } else {
-        const Fr w = twiddle(st, at.col);
-        v[1] = mont_mul_lazy(d0, w);
-        v[3] = mont_mul_lazy(d1, w);
+        v[1] = times(d0, st, at.col);
+        v[3] = times(d1, st, at.col);
       }
     }
     if (st + 2 < s) {

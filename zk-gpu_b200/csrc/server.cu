@@ -125,10 +125,9 @@ size_t Server::estimate_bytes(uint32_t log_m) const {
     return 4 * (3 * S + entries * 5 / 2 + S * xw + (heads + heads / 16 + 2) * (xw + 1) + 8 * W * B / 16 * xw / 8 +
                 (glv ? m * 16 : 0) + 4096);
   };
-  // scratch, twiddle words (both directions), staged twiddle tables (both directions: 40 bytes
-  // per element for the first pass, at most as much again for the later passes' small tables
-  // at these sizes) or the twiddle limbs of form 1 (20 bytes per element per direction)
-  const size_t ntt = 32 * N + 2 * 16 * N + 2 * 48 * N;
+  // scratch and pass twiddle tables (both directions: 64 bytes per element for the first pass, an
+  // eighth of that at most for the later passes' small tables at these sizes)
+  const size_t ntt = 32 * N + 2 * 72 * N;
   const size_t bufs = 3 * 32 * m + 32 * m + 3 * 32 * N + 4096;
   return msm(32) + msm(64) + ntt + bufs;
 }
