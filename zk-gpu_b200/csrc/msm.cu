@@ -36,14 +36,6 @@ static void set_acc_smem_limits() {
              "accumulation smem attribute");
 }
 
-// The last reduction level's block holds one XYZZ point per thread in shared memory: 64 KiB for
-// G2 (256 threads x 256 bytes), above the default limit.
-static void set_scan_smem_limits() {
-  const int bytes = (int)(kScanThreads * sizeof(Xyzz<Fq2CP>));
-  check_cuda(cudaFuncSetAttribute(msm_reduce_scan<Fq2CP>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes),
-             "reduction smem attribute");
-}
-
 uint32_t default_window(size_t n) {
   // clamp(log2(max(n,1)) - 5, 11, 16) (src/msm.rs:78-80)
   size_t v = n < 1 ? 1 : n;
@@ -78,7 +70,6 @@ MsmPlan::MsmPlan(zkg_ctx* c_, int group_, size_t n_, uint32_t c, uint32_t item_p
   use(ctx);
   if (group == ZKG_G2) {
     set_acc_smem_limits();
-    set_scan_smem_limits();
   }
   glv = glv_default();
   // The plan's own choice, form 4 for G1 and form 2 for G2: integer products with interleaved
@@ -137,12 +128,11 @@ void MsmPlan::layout() {
   buckets.alloc(slots * xw, "msm buckets");
 
   heads_max = (max_entries + seg_len - 1) / seg_len;
-  // Chains of the merge and running-sum levels. Merge: 4 heads per thread (twice the levels of
-  // 16, a quarter of the chain; measured faster at every size, G1 2^24 1.43 -> 1.05 ms). Running
-  // sums: chunks of 4 buckets below 2^23 entries, 8 above (measured: reduce + window sums at
-  // G1 2^24 1.30 / 1.20 / 1.25 ms for chunks of 4 / 8 / 16, at 2^16 0.47 / 0.52 / 0.65 ms).
+  // Merge: 4 heads per thread (twice the levels of 16, a quarter of the chain; measured faster at
+  // every size, G1 2^24 1.43 -> 1.05 ms). Running sums: the fewest buckets per thread that leave one
+  // chunked level before the marginals, at most 8.
   merge_fan_in = 4;
-  const uint32_t chunk_log = (double)max_entries < (double)(1u << 23) ? 2 : 3;
+  const uint32_t chunk_log = half > 4 * kMarginalMax ? 3 : half > 2 * kMarginalMax ? 2 : 1;
   size_t len = heads_max;
   merge_levels = 0;
   while (len > 1) {
@@ -155,26 +145,19 @@ void MsmPlan::layout() {
   heads[1].alloc(std::max<size_t>(second, 1) * xw, "msm heads");
   head_keys[1].alloc(std::max<size_t>(second, 1), "msm head keys");
 
-  // Running-sum levels: m_0 = B; m_{l+1} = ceil(m_l / C) - 1 while positive (C = 2^chunk_log).
+  // Running-sum levels: m_0 = B; m_{l+1} = ceil(m_l / C) - 1 (C = 2^chunk_log) down to at most
+  // kMarginalMax values, the last level's (level_m.back()).
   std::memset(&levels, 0, sizeof(levels));
   levels.chunk_log = chunk_log;
   const uint32_t bucket_chunk = 1u << chunk_log;
   uint32_t m = half;
   size_t tot_points = 0, run_points = 0;
-  std::vector<uint32_t> ms;
-  while (m > 0) {
+  level_m.clear();
+  while (m > kMarginalMax) {
     if (levels.count >= (uint32_t)kMaxReduceLevels) fail(ZKG_EINVAL, "too many reduction levels");
-    if (m <= kScanLevelMax) {  // the last level: one block per window sums it whole (msm_reduce_scan)
-      ms.push_back(m);
-      levels.tot_len[levels.count] = 1;
-      levels.tot_offset[levels.count] = (uint32_t)tot_points;
-      tot_points += windows;
-      levels.count++;
-      break;
-    }
-    uint32_t chunks = (m + bucket_chunk - 1) / bucket_chunk;
-    uint32_t blocks = (chunks + kReduceThreads - 1) / kReduceThreads;  // one tot point per block
-    ms.push_back(m);
+    const uint32_t chunks = (m + bucket_chunk - 1) / bucket_chunk;
+    const uint32_t blocks = (chunks + kReduceThreads - 1) / kReduceThreads;  // one tot point per block
+    level_m.push_back(m);
     levels.tot_len[levels.count] = blocks;
     levels.tot_offset[levels.count] = (uint32_t)tot_points;
     tot_points += (size_t)blocks * windows;
@@ -182,10 +165,17 @@ void MsmPlan::layout() {
     levels.count++;
     run_points = std::max<size_t>(run_points, (size_t)m * windows);
   }
-  level_m = ms;
-  tots.alloc(tot_points * xw, "msm tots");
+  level_m.push_back(m);
+  uint32_t bits = 0;
+  while ((1u << bits) < m) bits++;
+  marg_lo = (bits + 1) / 2;
+  marg_hi = bits - marg_lo;
+  marg_stride = (1u << marg_lo) + (1u << marg_hi) + levels.count;
+  tots.alloc(std::max<size_t>(tot_points, 1) * xw, "msm tots");
   runs[0].alloc(std::max<size_t>(run_points, 1) * xw, "msm runs");
   runs[1].alloc(std::max<size_t>(run_points, 1) * xw, "msm runs");
+  marginals.alloc((size_t)windows * marg_stride * xw, "msm marginals");
+  bit_sums.alloc((size_t)windows * (bits + 1) * xw, "msm bit sums");
   window_sums.alloc((size_t)windows * xw, "msm window sums");
   if (glv) glv_bases.alloc(chunk * affine_words(), "msm GLV bases (phi)");
   else glv_bases.release();
@@ -371,9 +361,8 @@ void MsmPlan::stage(int which, const uint32_t* bases, const uint32_t* scalars, c
       break;
     }
     case kStageCombine:
-      // c (W - 1) dependent doublings: one warp, each level's independent products on separate
-      // lanes. G1 inlines its products (measured 5-8% faster than one out-of-line product per
-      // lane: 2^16 with GLV 0.287 -> 0.265 ms); G2 keeps the out-of-line Fq2 products.
+      // c (W - 1) dependent doublings: one group of lanes, each level's independent products on
+      // separate lanes (curve_lanes.cuh).
       if constexpr (std::is_same<F, Fq>::value)
         msm_combine_lanes<Fq><<<1, 32, 0, s>>>(window_sums.ptr, active_windows(), glv ? 128u / windows : c,
                                                glv ? 128u % windows : 0u, combine_out);
@@ -428,13 +417,6 @@ void MsmPlan::tail_stage(int which, cudaStream_t s) {
       uint32_t in_stride = half;
       for (uint32_t l = 0; l < levels.count; l++) {
         uint32_t m = level_m[l];
-        if (m <= kScanLevelMax) {  // the last level
-          msm_reduce_scan<FC><<<active_windows(), kScanThreads, kScanThreads * sizeof(Xyzz<FC>), s>>>(
-              in, in_stride, m, l == 0 ? slot_start.ptr : nullptr, tots.ptr + (size_t)levels.tot_offset[l] * xyzz_words(),
-              levels.tot_len[l]);
-          check_launch("msm_reduce_scan");
-          break;
-        }
         uint32_t chunks = (m + (1u << levels.chunk_log) - 1) >> levels.chunk_log;
         uint32_t* run_out = runs[l & 1].ptr;
         const dim3 grid(levels.tot_len[l], active_windows());
@@ -449,10 +431,21 @@ void MsmPlan::tail_stage(int which, cudaStream_t s) {
       break;
     }
     case kStageWindows: {
-      msm_window_sums<FC><<<active_windows(), kWindowThreads, kWindowThreads * sizeof(Xyzz<FC>), s>>>(tots.ptr,
-                                                                                                    levels,
-                                                                                            window_sums.ptr);
-      check_launch("msm_window_sums");
+      // the last level's vector: the buckets, or the last chunked level's running sums
+      const uint32_t l = levels.count, m = level_m[l];
+      const uint32_t* in = l == 0 ? buckets.ptr : runs[(l - 1) & 1].ptr;
+      const uint32_t rows = (m + (1u << marg_lo) - 1) >> marg_lo, threads = SubsetThreads<FC>::value;
+      msm_marginals<FC><<<dim3((1u << marg_lo) + rows + l, active_windows()), threads, 0, s>>>(
+          in, l == 0 ? half : m, m, marg_lo, l == 0 ? slot_start.ptr : nullptr, tots.ptr, levels, marginals.ptr,
+          marg_stride);
+      check_launch("msm_marginals");
+      msm_bit_sums<FC><<<dim3(marg_lo + marg_hi + 1, active_windows()), threads, 0, s>>>(
+          marginals.ptr, marg_stride, m, marg_lo, marg_hi, bit_sums.ptr);
+      check_launch("msm_bit_sums");
+      msm_window_fold<FC><<<active_windows(), kFoldGroups * LaneGroup<FC>::kLanes, 0, s>>>(
+          bit_sums.ptr, marg_lo + marg_hi, marginals.ptr + ((size_t)(1u << marg_lo) + rows) * xyzz_words(), marg_stride, l,
+          levels.chunk_log, window_sums.ptr);
+      check_launch("msm_window_fold");
       break;
     }
     case kStageCombine:  // launched by stage() (msm_combine_lanes)

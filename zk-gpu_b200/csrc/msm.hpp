@@ -87,6 +87,8 @@ struct MsmPlan {
   DeviceArray ranks, digits;  // the ranked sort's rank (32 bits) and digit (16 bits) per (window, point), window-major
   DeviceArray glv_bases;      // GLV mode: phi(P_0)..phi(P_{n-1})
   DeviceArray heads[2], head_keys[2];
+  uint32_t marg_lo = 0, marg_hi = 0, marg_stride = 0;  // the last level's column and row bits (msm_marginals)
+  DeviceArray marginals, bit_sums;
   DeviceArray tots, runs[2], window_sums, result, partial;  // partial: a later pass's result
   zkg_buf result_handle;
   StageTimer timer;

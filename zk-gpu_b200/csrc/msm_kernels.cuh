@@ -19,13 +19,12 @@
 //                       L1 of them, adds runs that start in its range into the bucket, and
 //                       passes runs that continue from the previous range to the next level
 //                       (log_L1 levels)                            [msm_merge/finalize.wgsl]
-//   6. reduce levels    per window S_w = sum_b (b+1) * bucket_b, by chunked running sums:
-//                       chunk k of 16 buckets gives tot_k = sum_j (j+1) B_j and run_k =
-//                       sum_j B_j; S_w = sum_k tot_k + 16 * sum_k k * run_k, and the second
-//                       sum is the same problem over run_1.. (next level)
-//                                                                  [msm_reduce_chunks.wgsl,
-//                                                                   msm_sum.wgsl]
-//   7. window sums      per window, sum each level's tot_k and fold levels (x16 between)
+//   6. reduce level     per window S_w = sum_b (b+1) * bucket_b; above 4096 buckets by chunked
+//                       running sums: chunk k of C buckets gives tot_k = sum_j (j+1) B_j and
+//                       run_k = sum_j B_j; S_w = sum_k tot_k + C * sum_k k * run_k, and the
+//                       second sum is the same problem over run_1.. [msm_reduce_chunks.wgsl]
+//   7. window sums      per window the last vector's columns and rows, their bits' sums, and the
+//                       fold of those by doublings                [msm_sum.wgsl]
 //   8. combine          Horner over windows, c doublings each      [msm_combine.wgsl]
 #pragma once
 #include "curve.cuh"
@@ -845,20 +844,29 @@ __global__ void __launch_bounds__(kMergeTailThreads) msm_merge_tail(const uint32
 
 // ------------------------------------------------------------------ bucket reduction
 
-// Block-wide sum of XYZZ values (one per thread) through shared memory.
+// Sum of the n points (a power of two) in shared memory at sh, left in sh[0], by the whole block:
+// halving levels, a thread per addition while there are at least kThreadAdds of them (G1; an Fq2
+// addition takes a thread 18 us), a group of lanes per addition below (2 us, 2.6 us for G2, where a
+// thread takes 6).
 template <class F>
-__device__ Xyzz<F> block_sum(Xyzz<F> v, Xyzz<F>* sh) {
-  sh[threadIdx.x] = v;
-  __syncthreads();
-  for (unsigned stride = blockDim.x / 2; stride > 0; stride >>= 1) {
-    if (threadIdx.x < stride) sh[threadIdx.x] = xyzz_add(sh[threadIdx.x], sh[threadIdx.x + stride]);
+__device__ __forceinline__ void tree_sum(uint32_t* sh, uint32_t n) {
+  constexpr int XW = PointWords<F>::xyzz;
+  constexpr uint32_t kThreadAdds = XW == 32 ? 16 : 64;
+  const uint32_t groups = blockDim.x / LaneGroup<F>::kLanes, group = threadIdx.x / LaneGroup<F>::kLanes;
+  for (uint32_t h = n / 2; h >= 1; h >>= 1) {
+    if (h >= kThreadAdds) {
+      for (uint32_t i = threadIdx.x; i < h; i += blockDim.x)
+        store_xyzz(sh + (size_t)i * XW, xyzz_add(load_xyzz<F>(sh + (size_t)i * XW), load_xyzz<F>(sh + (size_t)(i + h) * XW)));
+    } else {
+      for (uint32_t i0 = 0; i0 < h; i0 += groups) {
+        const uint32_t i = i0 + group;
+        const bool active = i < h;
+        lane_add<F>(sh + (active ? i : 0) * XW, sh + (active ? i + h : 0) * XW, sh + (active ? i : 0) * XW, active);
+      }
+    }
     __syncthreads();
   }
-  Xyzz<F> r = sh[0];
-  __syncthreads();
-  return r;
 }
-
 
 // Level of the running-sum reduction. Per window w the input holds m values A_0..A_{m-1} at
 // in + (w * in_stride + b) * XW; level 0 reads the buckets, where an empty slot (no entries)
@@ -874,8 +882,7 @@ __global__ void __launch_bounds__(kReduceThreads) msm_reduce_level(const uint32_
                                                                    uint32_t* __restrict__ tot_out, uint32_t tot_stride,
                                                                    uint32_t* __restrict__ run_out, uint32_t run_stride) {
   constexpr int XW = PointWords<F>::xyzz;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Xyzz<F>* sh = reinterpret_cast<Xyzz<F>*>(smem_raw);
+  extern __shared__ __align__(16) uint32_t sh_words[];
   const uint32_t chunk = 1u << chunk_log;
   const uint32_t chunks = (m + chunk - 1) / chunk;
   const uint32_t w = blockIdx.y, j = blockIdx.x;
@@ -891,98 +898,195 @@ __global__ void __launch_bounds__(kReduceThreads) msm_reduce_level(const uint32_
     }
     if (k >= 1) store_xyzz(run_out + ((size_t)w * run_stride + k - 1) * XW, run);
   }
-  tot = block_sum(tot, sh);
-  if (threadIdx.x == 0) store_xyzz(tot_out + ((size_t)w * tot_stride + j) * XW, tot);
+  store_xyzz(sh_words + threadIdx.x * XW, tot);
+  __syncthreads();
+  tree_sum<F>(sh_words, kReduceThreads);
+  if (threadIdx.x < XW) tot_out[((size_t)w * tot_stride + j) * XW + threadIdx.x] = sh_words[threadIdx.x];
 }
 
 
-// The last level: S = sum_b (b + 1) A_b over m <= kScanLevelMax values per window in one block
-// (grid: windows). Thread t owns K = m_pad / 256 consecutive values (K a power of two, at most 4)
-// and forms ls_t = sum_j (j + 1) A_{Kt+j} and lt_t = sum_j A_{Kt+j}; then S = sum_t ls_t +
-// K sum_{t >= 1} suf_t with suf_t = sum_{u >= t} lt_u, a suffix scan over the threads (Hillis-
-// Steele in shared memory) followed by one block sum: about 2K + 2 log2(256) + 2 dependent
-// additions, where further chunked levels would each add a chain and a block sum.
-template <class F>
-__global__ void __launch_bounds__(kScanThreads) msm_reduce_scan(const uint32_t* __restrict__ in, uint32_t in_stride,
-                                                                uint32_t m, const uint32_t* __restrict__ slot_start,
-                                                                uint32_t* __restrict__ tot_out, uint32_t tot_stride) {
-  constexpr int XW = PointWords<F>::xyzz;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Xyzz<F>* sh = reinterpret_cast<Xyzz<F>*>(smem_raw);
-  const uint32_t w = blockIdx.x, t = threadIdx.x;
-  uint32_t k = 1;
-  while (k * kScanThreads < m) k <<= 1;
-  Xyzz<F> run = xyzz_infinity<F>(), ls = xyzz_infinity<F>();
-  for (uint32_t j = k; j-- > 0;) {
-    const uint32_t b = t * k + j;
-    if (b >= m) continue;
-    const size_t slot = (size_t)w * in_stride + b;
-    const bool empty = slot_start && __ldg(&slot_start[slot]) == __ldg(&slot_start[slot + 1]);
-    if (!empty) run = xyzz_add(run, load_xyzz<F>(in + slot * XW));
-    ls = xyzz_add(ls, run);
-  }
-  // suffix sums of the threads' totals
-  Xyzz<F> suf = run;
-  sh[t] = suf;
-  __syncthreads();
-  for (uint32_t d = 1; d < kScanThreads; d <<= 1) {
-    const Xyzz<F> other = t + d < kScanThreads ? sh[t + d] : xyzz_infinity<F>();
-    __syncthreads();
-    suf = xyzz_add(suf, other);
-    sh[t] = suf;
-    __syncthreads();
-  }
-  Xyzz<F> next = t + 1 < kScanThreads ? sh[t + 1] : xyzz_infinity<F>();
-  __syncthreads();
-  for (uint32_t kk = k; kk > 1; kk >>= 1) next = xyzz_double(next);  // K suf_{t+1}
-  const Xyzz<F> total = block_sum(xyzz_add(ls, next), sh);
-  if (t == 0) store_xyzz(tot_out + (size_t)w * tot_stride * XW, total);
-}
-
-// One block per window: S_w = sum over levels l of C^l * sum_k tot_l[k] (C = 2^chunk_log),
-// folded from the top level down (chunk_log doublings per level) by warp 0 with lane-parallel
-// products.
-template <class F>
-__global__ void __launch_bounds__(kWindowThreads) msm_window_sums(const uint32_t* __restrict__ tots, ReduceLevels lv,
-                                                                  uint32_t* __restrict__ window_sums) {
-  constexpr int XW = PointWords<F>::xyzz;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Xyzz<F>* sh = reinterpret_cast<Xyzz<F>*>(smem_raw);
-  __shared__ uint32_t scratch[32 * 8];
-  const LaneScratch sm{scratch};
-  const uint32_t w = blockIdx.x;
-  Xyzz<F> acc = xyzz_infinity<F>();
-  for (int l = (int)lv.count - 1; l >= 0; l--) {
-    Xyzz<F> part = xyzz_infinity<F>();
-    const uint32_t* base = tots + ((size_t)lv.tot_offset[l] + (size_t)w * lv.tot_len[l]) * XW;
-    for (uint32_t k = threadIdx.x; k < lv.tot_len[l]; k += blockDim.x) part = xyzz_add(part, load_xyzz<F>(base + (size_t)k * XW));
-    part = block_sum(part, sh);
-    if (threadIdx.x < 32) {  // warp 0 folds the levels, products of a level on separate lanes
-      for (uint32_t d = 0; d < lv.chunk_log; d++) acc = lane_double(acc, sm);  // x chunk
-      acc = lane_add(acc, part, sm);
+// The last level: S = sum_i (i + 1) A_i over m <= kMarginalMax values per window, by marginals. With i =
+// l + 2^lo h, sum_i i A_i = sum_l l C_l + 2^lo sum_h h R_h, C_l the sum of column l and R_h of row h; and
+// over the bits of l, sum_l l C_l = sum_k 2^k Z_k, Z_k the sum of the C_l whose l has bit k, likewise for
+// h. So three launches: the columns and rows (each at most 64 values), the Z_k and sum_l C_l (at most 32
+// columns or rows each), and the fold. All are trees, about log2(64) + log2(32) additions deep where
+// running sums and a suffix scan over 256 threads made 26 additions, on one SM per window.
+//
+// A sum of points that a block forms: which values of a window's vector, and how many.
+enum SubsetKind : uint32_t { kColumn, kRow, kBit, kAll };
+struct Subset {
+  SubsetKind kind;
+  uint32_t arg, lo, m;  // column l, row h or bit k; columns = 2^lo; the vector's length
+  __device__ __forceinline__ uint32_t size() const {
+    const uint32_t cols = 1u << lo;
+    switch (kind) {
+      case kColumn: return arg < m ? (m - arg + cols - 1) >> lo : 0;
+      case kRow: return min(cols, m - min(m, arg << lo));
+      case kBit: {  // indices below m with bit arg set
+        const uint32_t full = m >> (arg + 1), rest = m & ((2u << arg) - 1);
+        return (full << arg) + (rest > (1u << arg) ? rest - (1u << arg) : 0);
+      }
+      default: return m;
     }
   }
-  if (threadIdx.x == 0) store_xyzz(window_sums + (size_t)w * XW, acc);
+  __device__ __forceinline__ uint32_t index(uint32_t e) const {
+    switch (kind) {
+      case kColumn: return arg + (e << lo);
+      case kRow: return (arg << lo) + e;
+      case kBit: return ((e >> arg) << (arg + 1)) | (1u << arg) | (e & ((1u << arg) - 1));
+      default: return e;
+    }
+  }
+};
+
+// *out = the sum over the subset of the window's vector at `in`; a value whose slot is empty
+// (slot_start, when given, has the window's slots) is the point at infinity. One block.
+template <class F>
+__device__ __forceinline__ void subset_sum(const Subset& s, const uint32_t* __restrict__ in,
+                                           const uint32_t* __restrict__ slot_start, uint32_t* __restrict__ out,
+                                           uint32_t* sh) {
+  constexpr int XW = PointWords<F>::xyzz;
+  const uint32_t size = s.size();
+  uint32_t n = 1;
+  while (n < size && n < blockDim.x) n <<= 1;
+  if (threadIdx.x < n) {
+    Xyzz<F> v = xyzz_infinity<F>();
+    for (uint32_t e = threadIdx.x; e < size; e += n) {
+      const uint32_t i = s.index(e);
+      if (slot_start && __ldg(&slot_start[i]) == __ldg(&slot_start[i + 1])) continue;
+      v = xyzz_add(v, load_xyzz<F>(in + (size_t)i * XW));
+    }
+    store_xyzz(sh + (size_t)threadIdx.x * XW, v);
+  }
+  __syncthreads();
+  tree_sum<F>(sh, n);
+  if (threadIdx.x < XW) out[threadIdx.x] = sh[threadIdx.x];
+  if (XW > blockDim.x && threadIdx.x + blockDim.x < XW) out[threadIdx.x + blockDim.x] = sh[threadIdx.x + blockDim.x];
 }
 
-// result = sum_w 2^(pos_w) S_w by Horner from the top window (msm_combine.wgsl:13-22), by one
-// warp: each level's independent products run on separate lanes (curve_lanes.cuh). Window w is
-// `base` bits wide, or base + 1 for w < extra (pos_w is the sum of the widths below w): base =
-// c, extra = 0 for the plain windows, the glv_window_width split for GLV. F is the
-// one-product-per-call form (FqC or Fq2C).
+// Threads of a subset's block: one warp for G1 (a window has at least 64 subsets), four for G2, whose
+// additions take sixteen lanes.
+template <class F>
+struct SubsetThreads {
+  static constexpr uint32_t value = PointWords<F>::xyzz == 32 ? 32 : 128;
+};
+
+// Grid (2^lo + rows + lv.count, windows): the columns and rows of the last level's vector, and each
+// chunked level's block totals summed up; a window's results at marg + w * marg_stride points, columns
+// first, then rows, then the levels.
+template <class F>
+__global__ void __launch_bounds__(SubsetThreads<F>::value)
+    msm_marginals(const uint32_t* __restrict__ in, uint32_t in_stride, uint32_t m, uint32_t lo,
+                  const uint32_t* __restrict__ slot_start, const uint32_t* __restrict__ tots, ReduceLevels lv,
+                  uint32_t* __restrict__ marg, uint32_t marg_stride) {
+  constexpr int XW = PointWords<F>::xyzz;
+  __shared__ __align__(16) uint32_t sh[SubsetThreads<F>::value * XW];
+  const uint32_t w = blockIdx.y, j = blockIdx.x, cols = 1u << lo, rows = (m + cols - 1) >> lo;
+  uint32_t* const out = marg + ((size_t)w * marg_stride + j) * XW;
+  if (j >= cols + rows) {
+    const uint32_t l = j - cols - rows;
+    subset_sum<F>(Subset{kAll, 0, 0, lv.tot_len[l]}, tots + ((size_t)lv.tot_offset[l] + (size_t)w * lv.tot_len[l]) * XW,
+                  nullptr, out, sh);
+    return;
+  }
+  subset_sum<F>(j < cols ? Subset{kColumn, j, lo, m} : Subset{kRow, j - cols, lo, m}, in + (size_t)w * in_stride * XW,
+                slot_start ? slot_start + (size_t)w * in_stride : nullptr, out, sh);
+}
+
+// Grid (lo + hi + 1, windows): Z_k of the columns' bits, then of the rows', then the sum of all columns.
+template <class F>
+__global__ void __launch_bounds__(SubsetThreads<F>::value)
+    msm_bit_sums(const uint32_t* __restrict__ marg, uint32_t marg_stride, uint32_t m, uint32_t lo, uint32_t hi,
+                 uint32_t* __restrict__ bits) {
+  constexpr int XW = PointWords<F>::xyzz;
+  __shared__ __align__(16) uint32_t sh[SubsetThreads<F>::value * XW];
+  const uint32_t w = blockIdx.y, k = blockIdx.x, cols = 1u << lo, rows = (m + cols - 1) >> lo;
+  const uint32_t* const columns = marg + (size_t)w * marg_stride * XW;
+  const bool high = k >= lo && k < lo + hi;
+  const Subset s = k < lo ? Subset{kBit, k, 0, cols} : high ? Subset{kBit, k - lo, 0, rows} : Subset{kAll, 0, 0, cols};
+  subset_sum<F>(s, high ? columns + (size_t)cols * XW : columns, nullptr, bits + ((size_t)w * (lo + hi + 1) + k) * XW, sh);
+}
+
+// S_w from the Z_k: kFoldGroups groups of lanes run Horner over a share of the bits each, the first
+// folds the shares and adds the sum of all values; then for each chunked level, from the last one
+// down, S = 2^chunk_log S + its total.
+constexpr uint32_t kFoldGroups = 4;
+template <class F>
+__global__ void __launch_bounds__(kFoldGroups * LaneGroup<F>::kLanes)
+    msm_window_fold(const uint32_t* __restrict__ bits, uint32_t bit_count, const uint32_t* __restrict__ totals,
+                    uint32_t totals_stride, uint32_t levels, uint32_t chunk_log, uint32_t* __restrict__ window_sums) {
+  constexpr int XW = PointWords<F>::xyzz;
+  __shared__ __align__(16) uint32_t share[kFoldGroups][XW];
+  __shared__ __align__(16) uint32_t none[XW];  // the point at infinity
+  const uint32_t w = blockIdx.x, group = threadIdx.x / LaneGroup<F>::kLanes;
+  const unsigned role = lane_role<F>();
+  const uint32_t* const z = bits + (size_t)w * (bit_count + 1) * XW;
+  const uint32_t per = (bit_count + kFoldGroups - 1) / kFoldGroups, first = group * per;
+  for (uint32_t i = threadIdx.x; i < XW; i += blockDim.x) none[i] = 0;
+  __syncthreads();
+  auto bit = [&](uint32_t k) { return k < bit_count ? z + (size_t)k * XW : none; };
+  uint32_t* const mine = share[group];
+  LanePoint<F> acc = lane_load<F>(bit(first + per - 1));
+  for (uint32_t k = per - 1; k-- > 0;) {
+    acc = lane_double(acc, role);
+    lane_store(mine, acc);
+    __syncwarp();
+    lane_add<F>(mine, bit(first + k), mine, true);
+    __syncwarp();
+    acc = lane_load<F>(mine);
+    __syncwarp();
+  }
+  if (per == 1) lane_store(mine, acc);
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  const bool lead = group == 0;
+  uint32_t* const sum = share[kFoldGroups - 1];  // starts as the top share
+  auto fold = [&](const LanePoint<F>& start, uint32_t doublings, const uint32_t* add) {  // into sum
+    LanePoint<F> v = start;
+    for (uint32_t d = 0; d < doublings; d++) v = lane_double(v, role);
+    __syncwarp();
+    // the sum goes beside what it reads: `none`, which no later step needs
+    if (lead) lane_store(none, v);
+    __syncwarp();
+    lane_add<F>(none, add, sum, lead);
+    __syncwarp();
+  };
+  LanePoint<F> v = lane_load<F>(sum);
+  for (uint32_t g = kFoldGroups - 1; g-- > 0;) {
+    fold(v, per, share[g]);
+    v = lane_load<F>(sum);
+  }
+  fold(v, 0, z + (size_t)bit_count * XW);
+  for (uint32_t l = levels; l-- > 0;) {
+    v = lane_load<F>(sum);
+    fold(v, chunk_log, totals + ((size_t)w * totals_stride + l) * XW);
+  }
+  for (uint32_t i = threadIdx.x; i < XW; i += 32) window_sums[(size_t)w * XW + i] = sum[i];
+}
+
+// result = sum_w 2^(pos_w) S_w by Horner from the top window (msm_combine.wgsl:13-22), by one group
+// of lanes (curve_lanes.cuh; the warp's other groups repeat its work). Window w is `base` bits wide,
+// or base + 1 for w < extra (pos_w is the sum of the widths below w): base = c, extra = 0 for the
+// plain windows, the glv_window_width split for GLV. Bound by the latency of the doublings' products.
 template <class F>
 __global__ void __launch_bounds__(32) msm_combine_lanes(const uint32_t* __restrict__ window_sums, uint32_t windows,
                                                         uint32_t base, uint32_t extra, uint32_t* __restrict__ result) {
-  __shared__ uint32_t scratch[32 * 8];
-  const LaneScratch sm{scratch};
   constexpr int XW = PointWords<F>::xyzz;
-  Xyzz<F> acc = load_xyzz<F>(window_sums + (size_t)(windows - 1) * XW);
+  __shared__ __align__(16) uint32_t sum[XW];
+  const bool first = threadIdx.x < LaneGroup<F>::kLanes;
+  const unsigned sm = lane_role<F>();
+  LanePoint<F> acc = lane_load<F>(window_sums + (size_t)(windows - 1) * XW);
   for (int w = (int)windows - 2; w >= 0; w--) {
     const uint32_t width = base + ((uint32_t)w < extra ? 1u : 0u);
     for (uint32_t k = 0; k < width; k++) acc = lane_double(acc, sm);
-    acc = lane_add(acc, load_xyzz<F>(window_sums + (size_t)w * XW), sm);
+    if (first) lane_store(sum, acc);
+    __syncwarp();
+    lane_add<F>(sum, window_sums + (size_t)w * XW, sum, first);
+    __syncwarp();
+    acc = lane_load<F>(sum);
+    __syncwarp();
   }
-  if (threadIdx.x == 0) store_xyzz(result, acc);
+  if (first) lane_store(result, acc);
 }
 
 // result <- result + partial (XYZZ, one thread): the passes of a run over more points than one
