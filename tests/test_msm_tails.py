@@ -47,3 +47,22 @@ def test_bucket_reduction(gpu, group, c):
         for glv in ((None, False) if group == "G1" else (None,)):
             got = gpu_msm(gpu, bases, scalars, (c, None), Group.G1 if group == "G1" else Group.G2, glv=glv)
             assert np.array_equal(got, want), (group, c, what, glv)
+
+
+@pytest.mark.parametrize("group", ["G1", "G2"])
+def test_long_runs_of_heads(gpu, group):
+    """One bucket, or a few, over many accumulation threads: runs of partial sums that end at, before
+    and after a merge tile's edge, fill several tiles, and continue through several levels."""
+    grp = Group.G1 if group == "G1" else Group.G2
+    aw = grp.affine_words()
+    tile = 256 if group == "G1" else 128
+    sizes = [2, 3, tile - 1, tile, tile + 1, 2 * tile + 1, 5 * tile + 7] + ([tile * tile + tile + 2] if group == "G1" else [])
+    pool = random_points(group, 41, max(sizes))
+    for n in sizes:
+        bases = pool[: aw * n]
+        for scalars in (np.tile(fr_words([1]), n), np.tile(fr_words([3, 3, 3, 1, 5]), n)[: 8 * n],
+                        np.concatenate([np.tile(fr_words([2]), n // 2), np.tile(fr_words([7]), n - n // 2)])):
+            want = msm_ref(group, bases, scalars)
+            for items in (1, 2, 3):
+                got = gpu_msm(gpu, bases, scalars, (9, items), grp)
+                assert np.array_equal(got, want), (group, n, items)

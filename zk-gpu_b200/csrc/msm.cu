@@ -46,17 +46,20 @@ uint32_t default_window(size_t n) {
   return (uint32_t)c;
 }
 
-// Points accumulated per thread when the caller does not choose, by the number of (point,
-// window) entries; measured on B200 (G1, uniform scalars, default windows with the GLV split,
-// sweeping 8..256): 2^16 points (1.6M entries) best at 32 (1.26 ms against 1.34 at 16: fewer
-// merge levels), 2^18 at 32, 2^20 at 64-128, 2^22 and 2^24 at 128; 2^14 at 8 (longer segments
-// lengthen the accumulation chains, shorter ones add heads and merge levels).
-static uint32_t auto_seg_len(size_t n, uint32_t windows) {
-  const double entries = (double)n * windows;
-  if (entries < (double)(1u << 19)) return 8;
-  if (entries < (double)(1u << 23)) return 32;
-  if (entries < (double)(1u << 26)) return 64;
-  return 128;
+// Points accumulated per thread when the caller does not choose. Long segments lengthen the chains of
+// additions, short ones add heads and merges: about 32 below 2^23 (window, point) entries, 64 below 2^26,
+// 128 above, and then as many as make the threads whole waves of the accumulation kernel (four blocks of
+// 128 an SM for G1, two for G2), whose last wave otherwise runs nearly empty: G2 2^18 4.75 ms at 32 points
+// (4.3 waves), 4.49 at 48 (2.9). Where 16 or fewer suffice, as many as leave one merge tile an SM (two
+// for G2), and at least 4: G1 2^14 0.488 ms at 8, 0.466 at 12.
+static uint32_t auto_seg_len(size_t n, uint32_t windows, int group, int sms) {
+  const size_t entries = n * windows, few = (size_t)sms * 256, wave = (size_t)sms * (group == ZKG_G1 ? 512 : 256);
+  const size_t small = (entries + few - 1) / few;
+  if (small <= 16) return (uint32_t)std::max<size_t>(small, 4);
+  const size_t target = entries < (size_t)1 << 23 ? 32 : entries < (size_t)1 << 26 ? 64 : 128;
+  const size_t waves = std::max<size_t>(1, (entries + wave * target / 2) / (wave * target));
+  if (waves > 16) return (uint32_t)target;  // a part of a wave in so many is nothing
+  return (uint32_t)((entries + wave * waves - 1) / (wave * waves));
 }
 
 MsmPlan::MsmPlan(zkg_ctx* c_, int group_, size_t n_, uint32_t c, uint32_t item_points)
@@ -110,7 +113,7 @@ void MsmPlan::layout() {
   windows = glv ? (128 + c - 1) / c : (255 + c - 1) / c;
   half = 1u << (c - 1);
   slots = (size_t)windows * half;
-  seg_len = item_points_req ? item_points_req : auto_seg_len(np, windows);
+  seg_len = item_points_req ? item_points_req : auto_seg_len(np, windows, group, ctx->sm_count);
   const size_t xw = xyzz_words();
   const size_t max_entries = (size_t)windows * np;
 
@@ -128,18 +131,13 @@ void MsmPlan::layout() {
   buckets.alloc(slots * xw, "msm buckets");
 
   heads_max = (max_entries + seg_len - 1) / seg_len;
-  // Merge: 4 heads per thread (twice the levels of 16, a quarter of the chain; measured faster at
-  // every size, G1 2^24 1.43 -> 1.05 ms). Running sums: the fewest buckets per thread that leave one
-  // chunked level before the marginals, at most 8.
-  merge_fan_in = 4;
+  // Running sums: the fewest buckets per thread that leave one chunked level before the marginals, at
+  // most 8.
   const uint32_t chunk_log = half > 4 * kMarginalMax ? 3 : half > 2 * kMarginalMax ? 2 : 1;
-  size_t len = heads_max;
+  const size_t tile = group == ZKG_G1 ? MergeTile<FqCP>::value : MergeTile<Fq2CP>::value;
   merge_levels = 0;
-  while (len > 1) {
-    len = (len + merge_fan_in - 1) / merge_fan_in;
-    merge_levels++;
-  }
-  size_t second = (heads_max + merge_fan_in - 1) / merge_fan_in;
+  for (size_t len = heads_max; len > 1; len = (len + tile - 1) / tile) merge_levels++;
+  const size_t second = (heads_max + tile - 1) / tile;
   heads[0].alloc(heads_max * xw, "msm heads");
   head_keys[0].alloc(heads_max, "msm head keys");
   heads[1].alloc(std::max<size_t>(second, 1) * xw, "msm heads");
@@ -391,24 +389,21 @@ template <class FC>
 void MsmPlan::tail_stage(int which, cudaStream_t s) {
   switch (which) {
     case kStageMerge: {
+      // `few`: a thread takes 6 us for an addition (G2 18), a group of lanes 2 (2.6) of which a block
+      // runs 16 (8) at once, so up to 48 (56) additions groups are the faster; 32 for G1 measured the
+      // same or better from 2^18 to 2^24, where threads do more of them per second
+      constexpr uint32_t tile = MergeTile<FC>::value;
+      const size_t smem = (size_t)tile * (sizeof(Xyzz<FC>) + 12);
       size_t len = heads_max;  // the largest a level can be (the entry count is on the device)
-      uint32_t l = 0;
-      for (; l < merge_levels; l++) {
-        size_t out_len = (len + merge_fan_in - 1) / merge_fan_in;
-        if (out_len <= kMergeTailThreads) break;  // the rest in one block (msm_merge_tail)
-        int src = l & 1, dst = src ^ 1;
-        msm_merge<FC><<<grid_for(out_len, 128), 128, 0, s>>>(slot_start.ptr, (uint32_t)active_slots(), seg_len, merge_fan_in, l,
-                                                            heads[src].ptr, head_keys[src].ptr, heads[dst].ptr,
-                                                            head_keys[dst].ptr, buckets.ptr);
+      for (uint32_t l = 0; l < merge_levels; l++) {
+        const size_t out_len = (len + tile - 1) / tile;
+        const int src = l & 1, dst = src ^ 1;
+        const uint32_t few = group == ZKG_G1 ? 32 : 56;
+        msm_merge<FC><<<(unsigned)out_len, kMergeThreads, smem, s>>>(slot_start.ptr, (uint32_t)active_slots(), seg_len, l, few,
+                                                                    heads[src].ptr, head_keys[src].ptr, heads[dst].ptr,
+                                                                    head_keys[dst].ptr, buckets.ptr);
         check_launch("msm_merge");
         len = out_len;
-      }
-      if (l < merge_levels) {
-        msm_merge_tail<FC><<<1, kMergeTailThreads, 0, s>>>(slot_start.ptr, (uint32_t)active_slots(), seg_len,
-                                                         merge_fan_in, l, merge_levels - l, heads[0].ptr,
-                                                         head_keys[0].ptr, heads[1].ptr, head_keys[1].ptr,
-                                                         buckets.ptr);
-        check_launch("msm_merge_tail");
       }
       break;
     }

@@ -79,7 +79,7 @@ struct MsmPlan {
   size_t active_slots() const { return fixed_base ? half : slots; }
   uint32_t active_windows() const { return fixed_base ? 1u : windows; }
   size_t slots = 0, heads_max = 0;
-  uint32_t merge_levels = 0, merge_fan_in = 16, scan_tiles_n = 0;
+  uint32_t merge_levels = 0, scan_tiles_n = 0;
   ReduceLevels levels;
   std::vector<uint32_t> level_m;
 

@@ -15,10 +15,10 @@
 //                       the parts of a bucket that continue into later segments ("heads")
 //                       are emitted per segment with the bucket's slot as key.
 //                                                                  [msm_accumulate.wgsl]
-//   5. merge levels     heads with equal keys are contiguous; each level sums runs of up to
-//                       L1 of them, adds runs that start in its range into the bucket, and
-//                       passes runs that continue from the previous range to the next level
-//                       (log_L1 levels)                            [msm_merge/finalize.wgsl]
+//   5. merge levels     heads with equal keys are contiguous; each level sums the runs within tiles
+//                       of 256 (G2: 128) of them, adds runs that start in a tile into the bucket,
+//                       and passes runs that continue from the previous tile to the next level
+//                                                                  [msm_merge/finalize.wgsl]
 //   6. reduce level     per window S_w = sum_b (b+1) * bucket_b; above 4096 buckets by chunked
 //                       running sums: chunk k of C buckets gives tot_k = sum_j (j+1) B_j and
 //                       run_k = sum_j B_j; S_w = sum_k tot_k + C * sum_k k * run_k, and the
@@ -749,97 +749,97 @@ __global__ void __launch_bounds__(128) msm_accumulate(const uint32_t* __restrict
 
 // ------------------------------------------------------------------ merge levels
 
+// Heads of one block (a tile): 256 for G1, 128 for G2 (32 KiB of points).
+template <class F>
+struct MergeTile {
+  static constexpr uint32_t value = PointWords<F>::xyzz == 32 ? 256 : 128;
+};
+constexpr uint32_t kMergeThreads = 128;
+
 // Length of the head array at merge level `level` (level 0 = the accumulate output).
-__device__ __forceinline__ uint32_t heads_len(uint32_t total, uint32_t seg_len, uint32_t fan_in, uint32_t level) {
+__device__ __forceinline__ uint32_t heads_len(uint32_t total, uint32_t seg_len, uint32_t tile, uint32_t level) {
   uint64_t len = ((uint64_t)total + seg_len - 1) / seg_len;
-  for (uint32_t l = 0; l < level; l++) len = (len + fan_in - 1) / fan_in;
+  for (uint32_t l = 0; l < level; l++) len = (len + tile - 1) / tile;
   return (uint32_t)len;
 }
 
+// One merge level: block u sums the runs of equal keys among heads [u T, u T + T). A run that starts
+// there is added into its bucket; one that continues from the tile before becomes head u of the next
+// level. One addition per bucket per level (only the tile where a run starts adds it), so a level
+// needs no atomics.
+//
+// Within a run the sum is a tree: at step d the heads at offsets that are multiples of 2d take the one d
+// further. Uniform scalars give runs of 4-5 heads, three steps; a bucket that fills the tile takes
+// log2 T. A step's additions go a thread each when they are many (more than `few`), else a group of
+// lanes each. Bound by the latency of the additions: the earlier levels of four heads per thread
+// needed eight launches of four to five additions in a row for 49152 heads, this needs two.
 template <class F>
-__device__ __forceinline__ void add_into_bucket(uint32_t* buckets, uint32_t key, const Xyzz<F>& v) {
+__global__ void __launch_bounds__(kMergeThreads) msm_merge(const uint32_t* __restrict__ slot_start, uint32_t num_slots,
+                                                           uint32_t seg_len, uint32_t level, uint32_t few,
+                                                           const uint32_t* __restrict__ in_pts,
+                                                           const uint32_t* __restrict__ in_keys,
+                                                           uint32_t* __restrict__ out_pts,
+                                                           uint32_t* __restrict__ out_keys,
+                                                           uint32_t* __restrict__ buckets) {
   constexpr int XW = PointWords<F>::xyzz;
-  uint32_t* b = buckets + (size_t)key * XW;
-  store_xyzz(b, xyzz_add(load_xyzz<F>(b), v));
-}
-
-// Thread u sums heads [u*f, u*f + f) of a level of len heads (f = fan_in). Runs that start
-// inside the range are added into their bucket; a run that continues from the previous range
-// becomes this thread's head for the next level. One add per bucket per level (only the range
-// where a run starts adds it), so a level needs no atomics.
-template <class F>
-__device__ __forceinline__ void merge_range(uint32_t u, uint32_t len, uint32_t fan_in, const uint32_t* __restrict__ in_pts,
-                                            const uint32_t* __restrict__ in_keys, uint32_t* __restrict__ out_pts,
-                                            uint32_t* __restrict__ out_keys, uint32_t* __restrict__ buckets) {
-  constexpr int XW = PointWords<F>::xyzz;
-  const uint64_t q0_64 = (uint64_t)u * fan_in;
-  if (q0_64 >= len) return;
-  const uint32_t q0 = (uint32_t)q0_64, q1 = min(q0 + fan_in, len);
-  const uint32_t prev = q0 > 0 ? in_keys[q0 - 1] : kNoKey;
-
-  uint32_t cur = kNoKey, start = q0, out_key = kNoKey;
-  Xyzz<F> acc = xyzz_infinity<F>();
-  for (uint32_t q = q0; q <= q1; q++) {
-    uint32_t k = q < q1 ? in_keys[q] : kNoKey;
-    if (k != cur || q == q1) {
-      if (cur != kNoKey) {
-        if (start == q0 && prev == cur) {
-          store_xyzz(out_pts + (size_t)u * XW, acc);
-          out_key = cur;
-        } else {
-          add_into_bucket<F>(buckets, cur, acc);
-        }
-      }
-      if (q == q1) break;
-      cur = k;
-      start = q;
-      acc = xyzz_infinity<F>();
-    }
-    if (k != kNoKey) acc = xyzz_add(acc, load_xyzz<F>(in_pts + (size_t)q * XW));
+  constexpr uint32_t T = MergeTile<F>::value, kGroups = kMergeThreads / LaneGroup<F>::kLanes;
+  extern __shared__ __align__(16) uint32_t merge_smem[];
+  uint32_t* const pts = merge_smem;        // [T] points
+  uint32_t* const keys = pts + T * XW;     // [T]
+  uint32_t* const offset = keys + T;       // [T] offset within the run
+  uint32_t* const work = offset + T;       // [T] the step's heads
+  __shared__ uint32_t work_count;
+  const uint32_t len = heads_len(__ldg(&slot_start[num_slots]), seg_len, T, level);
+  const uint32_t u = blockIdx.x, base = u * T;
+  if (len <= 1 || base >= len) return;  // the whole block
+  const uint32_t n = min(T, len - base), group = threadIdx.x / LaneGroup<F>::kLanes;
+  const uint32_t prev = base > 0 ? in_keys[base - 1] : kNoKey;
+  for (uint32_t i = threadIdx.x; i < n; i += kMergeThreads) {
+    const uint32_t k = in_keys[base + i];
+    keys[i] = k;
+    if (k != kNoKey) store_xyzz(pts + i * XW, load_xyzz<F>(in_pts + (size_t)(base + i) * XW));
   }
-  out_keys[u] = out_key;
-}
-
-// One merge level (grid over its output heads).
-template <class F>
-__global__ void __launch_bounds__(128) msm_merge(const uint32_t* __restrict__ slot_start, uint32_t num_slots,
-                                                 uint32_t seg_len, uint32_t fan_in, uint32_t level,
-                                                 const uint32_t* __restrict__ in_pts,
-                                                 const uint32_t* __restrict__ in_keys, uint32_t* __restrict__ out_pts,
-                                                 uint32_t* __restrict__ out_keys, uint32_t* __restrict__ buckets) {
-  const uint32_t total = __ldg(&slot_start[num_slots]);
-  const uint32_t len = heads_len(total, seg_len, fan_in, level);
-  if (len <= 1) return;  // nothing left to merge
-  merge_range<F>(blockIdx.x * blockDim.x + threadIdx.x, len, fan_in, in_pts, in_keys, out_pts, out_keys, buckets);
-}
-
-// The last merge levels, from first_level on, in one block of kMergeTailThreads: every such
-// level has at most kMergeTailThreads output heads (the host starts the tail where the largest
-// possible level fits), the levels run one after another with a block barrier between them
-// (the heads of a level are written by the block before the next reads them), and the
-// ping-pong buffers alternate by level parity as in msm_merge. The small late levels otherwise
-// cost a launch each (about 4-5 us) for a handful of heads.
-constexpr uint32_t kMergeTailThreads = 256;
-template <class F>
-__global__ void __launch_bounds__(kMergeTailThreads) msm_merge_tail(const uint32_t* __restrict__ slot_start,
-                                                                   uint32_t num_slots, uint32_t seg_len, uint32_t fan_in,
-                                                                   uint32_t first_level, uint32_t levels,
-                                                                   uint32_t* __restrict__ heads0,
-                                                                   uint32_t* __restrict__ keys0,
-                                                                   uint32_t* __restrict__ heads1,
-                                                                   uint32_t* __restrict__ keys1,
-                                                                   uint32_t* __restrict__ buckets) {
-  const uint32_t total = __ldg(&slot_start[num_slots]);
-  for (uint32_t l = first_level; l < first_level + levels; l++) {
-    const uint32_t len = heads_len(total, seg_len, fan_in, l);
-    if (len <= 1) break;  // uniform across the block
-    const bool odd = l & 1;
-    const uint32_t out_len = (len + fan_in - 1) / fan_in;
-    for (uint32_t u = threadIdx.x; u < out_len; u += blockDim.x)
-      merge_range<F>(u, len, fan_in, odd ? heads1 : heads0, odd ? keys1 : keys0, odd ? heads0 : heads1,
-                     odd ? keys0 : keys1, buckets);
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < n; i += kMergeThreads) {
+    uint32_t o = 0;
+    while (o < i && keys[i - o - 1] == keys[i]) o++;
+    offset[i] = o;
+  }
+  // work[0 .. work_count) = the heads i < n that `pick` takes
+  auto collect = [&](auto pick) {
     __syncthreads();
+    if (threadIdx.x == 0) work_count = 0;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < n; i += kMergeThreads)
+      if (keys[i] != kNoKey && pick(i)) work[atomicAdd(&work_count, 1u)] = i;
+    __syncthreads();
+    return work_count;
+  };
+  // target(i) += value(i) for the collected heads
+  auto add_all = [&](uint32_t count, auto target, auto value) {
+    if (count > few) {
+      for (uint32_t j = threadIdx.x; j < count; j += kMergeThreads) {
+        const uint32_t i = work[j];
+        store_xyzz(target(i), xyzz_add(load_xyzz<F>(target(i)), load_xyzz<F>(value(i))));
+      }
+    } else {
+      for (uint32_t j0 = 0; j0 < count; j0 += kGroups) {
+        const bool active = j0 + group < count;
+        const uint32_t i = work[active ? j0 + group : 0];
+        lane_add<F>(active ? target(i) : pts + i * XW, active ? value(i) : pts + i * XW, target(i), active);
+      }
+    }
+  };
+  for (uint32_t d = 1; d < T; d <<= 1) {
+    const uint32_t count = collect([&](uint32_t i) { return (offset[i] & (2 * d - 1)) == 0 && i + d < n && keys[i + d] == keys[i]; });
+    if (count == 0) break;  // no run is longer than d
+    add_all(count, [&](uint32_t i) { return pts + i * XW; }, [&](uint32_t i) { return pts + (i + d) * XW; });
   }
+  const bool continued = keys[0] != kNoKey && keys[0] == prev;
+  const uint32_t count = collect([&](uint32_t i) { return offset[i] == 0 && !(i == 0 && continued); });
+  add_all(count, [&](uint32_t i) { return buckets + (size_t)keys[i] * XW; }, [&](uint32_t i) { return pts + i * XW; });
+  if (continued && threadIdx.x < XW) out_pts[(size_t)u * XW + threadIdx.x] = pts[threadIdx.x];
+  if (threadIdx.x == 0) out_keys[u] = continued ? keys[0] : kNoKey;
 }
 
 // ------------------------------------------------------------------ bucket reduction
