@@ -76,10 +76,11 @@ MsmPlan::MsmPlan(zkg_ctx* c_, int group_, size_t n_, uint32_t c, uint32_t item_p
   }
   glv = glv_default();
   // The plan's own choice, form 4 for G1 and form 2 for G2: integer products with interleaved
-  // accumulators (field.cuh), inlined for G1 and two per out-of-line call for G2. Accumulation,
-  // ms: G1 2^16 / 2^20 / 2^22 0.30 / 2.80 / 9.72, against 0.32 / 2.96 / 10.28 for one product
-  // per call, 0.31 / 2.94 / 10.24 for two and 0.40 / 3.88 / 13.05 for double-precision limbs; G2
-  // 2^20 9.79, against 10.0 for one per call, 11.2 inlined and 17.3 for limbs.
+  // accumulators (field.cuh), inlined for G1; for G2 out of line, one reduction per component.
+  // Accumulation, ms: G1 2^16 / 2^20 / 2^22 0.30 / 2.80 / 9.72, against 0.32 / 2.96 / 10.28 for one
+  // product per call, 0.31 / 2.94 / 10.24 for two and 0.40 / 3.88 / 13.05 for double-precision
+  // limbs; G2 2^20 8.41, against 9.79 for pairs of reduced products, 9.79 for one product per call,
+  // 11.1 inlined and 17.3 for limbs (8.41 with two blocks an SM, 9.88 with three, which spill).
   acc_variant = group == ZKG_G1 ? 4 : 2;
   chunk = std::min(n, max_chunk());
   layout();
@@ -134,7 +135,7 @@ void MsmPlan::layout() {
   // Running sums: the fewest buckets per thread that leave one chunked level before the marginals, at
   // most 8.
   const uint32_t chunk_log = half > 4 * kMarginalMax ? 3 : half > 2 * kMarginalMax ? 2 : 1;
-  const size_t tile = group == ZKG_G1 ? MergeTile<FqCP>::value : MergeTile<Fq2CP>::value;
+  const size_t tile = group == ZKG_G1 ? MergeTile<FqCP>::value : MergeTile<Fq2L>::value;
   merge_levels = 0;
   for (size_t len = heads_max; len > 1; len = (len + tile - 1) / tile) merge_levels++;
   const size_t second = (heads_max + tile - 1) / tile;
@@ -377,9 +378,7 @@ void MsmPlan::stage(int which, const uint32_t* bases, const uint32_t* scalars, c
     case kStageMerge:
     case kStageReduce:
     case kStageWindows:
-      // Two products per out-of-line call in every form (measured faster than one per call for
-      // both groups, although the paired Fq2 kernels spill, and than inlined products for G1:
-      // 2^24 merge 1.10 -> 1.49 ms, reduce 0.66 -> 1.09 ms inlined).
+      // out-of-line products in every form (PairedOf)
       tail_stage<typename PairedOf<F>::type>(which, s);
       break;
   }

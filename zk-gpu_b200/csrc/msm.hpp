@@ -36,7 +36,8 @@ struct MsmPlan {
   size_t n;
   uint32_t c, windows = 0, half = 0, seg_len = 0;
   // Accumulation kernel form: 0 = integer field products inlined, 1 = through one out-of-line
-  // product, 2 = out of line, independent products two per call, 3 / 5 / 6 = bucket arithmetic in
+  // product, 2 = out of line, independent products two per call (G2: one reduction per component of
+  // an Fq2 product), 3 / 5 / 6 = bucket arithmetic in
   // double-precision limbs (msm_f64.cuh: two products per call, or for G1 the accumulator in
   // shared memory with one / two per call), 4 = for G1 the plan's own choice (inlined integer
   // products), for G2 limbs with one product per call. Every form fetches the next base into
