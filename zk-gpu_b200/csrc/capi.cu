@@ -472,7 +472,7 @@ int zkg_msm_params(const zkg_msm* msm, uint32_t* c, uint32_t* item_points, int* 
   return guard([&] {
     need(msm, "msm");
     if (c) *c = msm->plan.c;
-    if (item_points) *item_points = msm->plan.seg_len;
+    if (item_points) *item_points = msm->plan.segments().seg_len;
     if (variant) *variant = msm->plan.acc_variant;
   });
 }
@@ -684,7 +684,7 @@ int zkg_msm_last_entries(zkg_msm* msm, uint64_t* entries) {
     need(entries, "entries");
     use(msm->plan.ctx);
     uint32_t v = 0;
-    check_cuda(cudaMemcpyAsync(&v, msm->plan.slot_start.ptr + msm->plan.slots, 4, cudaMemcpyDeviceToHost,
+    check_cuda(cudaMemcpyAsync(&v, msm->plan.counts.ptr + msm->plan.active_slots(), 4, cudaMemcpyDeviceToHost,
                                msm->plan.ctx->stream),
                "entry count");
     check_cuda(cudaStreamSynchronize(msm->plan.ctx->stream), "entry count");

@@ -13,6 +13,7 @@
 
 #include "host_field.hpp"
 #include "msm.hpp"
+#include "msm_affine.cuh"
 #include "msm_f64.cuh"
 #include "msm_kernels.cuh"
 
@@ -52,8 +53,8 @@ uint32_t default_window(size_t n) {
 // 128 an SM for G1, two for G2), whose last wave otherwise runs nearly empty: G2 2^18 4.75 ms at 32 points
 // (4.3 waves), 4.49 at 48 (2.9). Where 16 or fewer suffice, as many as leave one merge tile an SM (two
 // for G2), and at least 4: G1 2^14 0.488 ms at 8, 0.466 at 12.
-static uint32_t auto_seg_len(size_t n, uint32_t windows, int group, int sms) {
-  const size_t entries = n * windows, few = (size_t)sms * 256, wave = (size_t)sms * (group == ZKG_G1 ? 512 : 256);
+uint32_t auto_seg_len(size_t entries, int group, int sms) {
+  const size_t few = (size_t)sms * 256, wave = (size_t)sms * (group == ZKG_G1 ? 512 : 256);
   const size_t small = (entries + few - 1) / few;
   if (small <= 16) return (uint32_t)std::max<size_t>(small, 4);
   const size_t target = entries < (size_t)1 << 23 ? 32 : entries < (size_t)1 << 26 ? 64 : 128;
@@ -62,8 +63,40 @@ static uint32_t auto_seg_len(size_t n, uint32_t windows, int group, int sms) {
   return (uint32_t)((entries + wave * waves - 1) / (wave * waves));
 }
 
-MsmPlan::MsmPlan(zkg_ctx* c_, int group_, size_t n_, uint32_t c, uint32_t item_points)
-    : ctx(c_), group(group_), n(n_), c(c) {
+// Entries of one batch of affine rounds. A batch's points between rounds take 48 bytes an entry (G2 96),
+// and there are two batches' scratch; G1 2^24 40.4 ms with batches of 2^24, 39.2 with 2^25.
+static size_t affine_batch(int group) { return (size_t)1 << (group == ZKG_G1 ? 25 : 24); }
+
+// Pairs per thread of a round over `pairs` pairs: about 32, such that the threads fill whole waves of
+// msm_affine_sums (four blocks an SM, two for G2) or, for small rounds, fewer down to 4.
+static uint32_t affine_per_thread(size_t pairs, int group, int sms) {
+  const size_t wave = (size_t)sms * (group == ZKG_G1 ? 4 : 2) * kAffineThreads;
+  const size_t waves = std::max<size_t>(1, (pairs + wave * 16) / (wave * 32));
+  return (uint32_t)std::max<size_t>(4, (pairs + wave * waves - 1) / (wave * waves));
+}
+
+// Rounds of affine additions for `entries` entries over the plan's slots (msm_affine.cuh). Each round
+// takes half of the additions that are left from the mixed to the cheaper affine form, but costs three
+// launches a batch, the latency of an inversion and half a group of padding a slot more. Accumulation and
+// merge, ms, with 0 / 2 / 3 / 4 rounds: G1 2^17 0.55 / 0.55 / 0.60 / 0.74, 2^18 0.92 / 0.82 / 0.89 / 1.12, 2^20
+// 2.96 / 2.54 / 2.53 / 2.94, 2^22 9.95 / 9.01 / 8.97 / 9.37, 2^24 39.0 / 35.3 / 34.2 / 33.9; G2 2^16 0.88 / 0.89 /
+// 1.01 / 1.44, 2^18 2.78 / 2.30 / 2.60 / 3.63, 2^20 8.73 / 7.12 / 7.90 / 11.5, 2^22 32.3 / 28.1 / 27.1. The
+// entries are the most there can be: sparse scalars (three in five zero digits) gain from larger sizes
+// on than uniform ones, so the line lies at 2^19 and G2 2^18 points (a sparse G1 MSM of 300007 points:
+// 1.01 ms without rounds, 1.09 with two).
+uint32_t MsmPlan::affine_rounds(size_t entries) const {
+  if (!affine) return 0;
+  const size_t per_slot = entries / slots;
+  uint32_t r = 0;
+  if (entries >= (size_t)1 << (group == ZKG_G1 ? 23 : 22) && per_slot >= 48) r = 2;
+  if (entries >= (size_t)1 << 26 && per_slot >= 128) r = 3;
+  if (entries >= (size_t)1 << 28 && per_slot >= 512) r = 4;
+  while (r > 0 && entries + slots * ((1u << r) - 1) > 0xfffffffeull) r--;  // places are 32-bit
+  return r;
+}
+
+MsmPlan::MsmPlan(zkg_ctx* c_, int group_, size_t n_, uint32_t c, uint32_t item_points, bool affine)
+    : ctx(c_), group(group_), n(n_), c(c), affine(affine) {
   if (n < 1) fail(ZKG_EINVAL, "an MSM needs at least one point");
   if (c < 9 || c > 20) fail(ZKG_EINVAL, "window size c must be in 9..=20, got " + std::to_string(c));
   if (group != ZKG_G1 && group != ZKG_G2) fail(ZKG_EINVAL, "group must be ZKG_G1 or ZKG_G2");
@@ -81,7 +114,7 @@ MsmPlan::MsmPlan(zkg_ctx* c_, int group_, size_t n_, uint32_t c, uint32_t item_p
   // product per call, 0.31 / 2.94 / 10.24 for two and 0.40 / 3.88 / 13.05 for double-precision
   // limbs; G2 2^20 8.41, against 9.79 for pairs of reduced products, 9.79 for one product per call,
   // 11.1 inlined and 17.3 for limbs (8.41 with two blocks an SM, 9.88 with three, which spill).
-  acc_variant = group == ZKG_G1 ? 4 : 2;
+  acc_variant = own_variant();
   chunk = std::min(n, max_chunk());
   layout();
   result.alloc(xyzz_words(), "msm result");
@@ -109,36 +142,85 @@ void MsmPlan::set_chunk(size_t points) {
   }
 }
 
+// Where the affine rounds' scratch does not fit the device beside the rest, the plan goes without.
 void MsmPlan::layout() {
-  const size_t np = glv ? 2 * chunk : chunk;  // points of the largest pass
+  const size_t np = glv ? 2 * chunk : chunk;
   windows = glv ? (128 + c - 1) / c : (255 + c - 1) / c;
   half = 1u << (c - 1);
   slots = (size_t)windows * half;
-  seg_len = item_points_req ? item_points_req : auto_seg_len(np, windows, group, ctx->sm_count);
+  if (const uint32_t group_log = affine_rounds(windows * np)) {
+    try {
+      layout_rounds(group_log);
+      return;
+    } catch (const Error& e) {
+      if (e.code != ZKG_ENOMEM) throw;
+      cudaGetLastError();
+    }
+  }
+  layout_rounds(0);
+}
+
+void MsmPlan::layout_rounds(uint32_t group_log) {
+  const size_t np = glv ? 2 * chunk : chunk;  // points of the largest pass
   const size_t xw = xyzz_words();
   const size_t max_entries = (size_t)windows * np;
-
-  counts.alloc(slots, "msm counts");
+  const size_t tile = group == ZKG_G1 ? MergeTile<FqCP>::value : MergeTile<Fq2L>::value;
+  auto segments_of = [&](uint32_t log) {
+    Segments g;
+    g.group_log = log;
+    g.groups = (max_entries + slots * (((size_t)1 << log) - 1)) >> log;  // at most: every slot's last group all but empty
+    g.seg_len = item_points_req ? item_points_req : auto_seg_len(g.groups, group, ctx->sm_count);
+    g.heads = (g.groups + g.seg_len - 1) / g.seg_len;
+    for (size_t len = g.heads; len > 1; len = (len + tile - 1) / tile) g.merge_levels++;
+    return g;
+  };
+  plain = segments_of(0);
+  rounds = segments_of(group_log);
+  counts.alloc(slots + 1, "msm counts");  // and the run's entry count
   slot_start.alloc(slots + 1, "msm slot_start");
   cursor.alloc(slots, "msm cursor");
   scan_tiles_n = (uint32_t)((slots + kScanTile - 1) / kScanTile);
   if (scan_tiles_n > (uint32_t)kScanTile) fail(ZKG_EINVAL, "too many bucket slots");
   tile_sums.alloc(scan_tiles_n, "msm scan tiles");
-  sorted.alloc(max_entries, "msm sorted");
+  sorted.alloc(rounds.groups << group_log, "msm sorted");
+  if (group_log) {
+    batch_groups = (uint32_t)std::min<size_t>((rounds.groups + 1) / 2, affine_batch(group) >> group_log);  // one for each stream
+    affine_sums.alloc(rounds.groups * affine_words(), "msm affine sums");
+    size_t threads = 0;  // of the largest round
+    for (uint32_t r = 1; r <= group_log; r++) {
+      const size_t pairs = (size_t)batch_groups << (group_log - r);
+      const size_t per = affine_per_thread(pairs, group, ctx->sm_count);
+      threads = std::max<size_t>(threads, (size_t)grid_for((pairs + per - 1) / per, kAffineThreads) * kAffineThreads);
+    }
+    for (AffineLane& lane : affine_lane) {
+      lane.inverses.alloc(threads * (affine_words() / 2), "msm affine inverses");
+      for (uint32_t k = 0; k < 2; k++) {  // rounds 1 and 2 write the largest arrays
+        if (group_log > k + 1)
+          lane.mid[k].alloc(((size_t)batch_groups << (group_log - 1 - k)) * affine_words(), "msm affine points");
+        else lane.mid[k].release();
+      }
+    }
+    if (!side.stream) check_cuda(cudaStreamCreateWithFlags(&side.stream, cudaStreamNonBlocking), "msm side stream");
+    if (!side.fork) check_cuda(cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming), "msm side event");
+    if (!side.join) check_cuda(cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming), "msm side event");
+  } else {
+    affine_sums.release();
+    for (AffineLane& lane : affine_lane) {
+      lane.inverses.release();
+      lane.mid[0].release();
+      lane.mid[1].release();
+    }
+  }
   if (c <= 16) {
     ranks.alloc(max_entries, "msm ranks");
     digits.alloc((max_entries + 1) / 2, "msm ranked digits");  // 16 bits per entry
   }
   buckets.alloc(slots * xw, "msm buckets");
 
-  heads_max = (max_entries + seg_len - 1) / seg_len;
   // Running sums: the fewest buckets per thread that leave one chunked level before the marginals, at
   // most 8.
   const uint32_t chunk_log = half > 4 * kMarginalMax ? 3 : half > 2 * kMarginalMax ? 2 : 1;
-  const size_t tile = group == ZKG_G1 ? MergeTile<FqCP>::value : MergeTile<Fq2L>::value;
-  merge_levels = 0;
-  for (size_t len = heads_max; len > 1; len = (len + tile - 1) / tile) merge_levels++;
-  const size_t second = (heads_max + tile - 1) / tile;
+  const size_t heads_max = std::max(plain.heads, rounds.heads), second = (heads_max + tile - 1) / tile;
   heads[0].alloc(heads_max * xw, "msm heads");
   head_keys[0].alloc(heads_max, "msm head keys");
   heads[1].alloc(std::max<size_t>(second, 1) * xw, "msm heads");
@@ -275,9 +357,10 @@ void MsmPlan::rank(const uint32_t* bases, const uint32_t* scalars, cudaStream_t 
 template <class F>
 void MsmPlan::stage(int which, const uint32_t* bases, const uint32_t* scalars, cudaStream_t s) {
   const unsigned b256 = 256;
+  const Segments& seg = segments();
   switch (which) {
     case kStageCount:
-      check_cuda(cudaMemsetAsync(counts.ptr, 0, active_slots() * 4, s), "msm counts clear");
+      check_cuda(cudaMemsetAsync(counts.ptr, 0, (active_slots() + 1) * 4, s), "msm counts clear");
       if (ranked_sort()) {
         if (sort_agg == 0)
           rank<0>(bases, scalars, s);
@@ -302,12 +385,12 @@ void MsmPlan::stage(int which, const uint32_t* bases, const uint32_t* scalars, c
     {
       const size_t ns = active_slots();
       const uint32_t tiles = (uint32_t)((ns + kScanTile - 1) / kScanTile);
-      scan_tile_sums<<<tiles, kScanBlock, 0, s>>>(counts.ptr, ns, tile_sums.ptr);
+      scan_tile_sums<<<tiles, kScanBlock, 0, s>>>(counts.ptr, ns, seg.group_log, tile_sums.ptr, counts.ptr + ns);
       check_launch("scan_tile_sums");
       scan_tiles<<<1, kScanBlock, 0, s>>>(tile_sums.ptr, tiles, slot_start.ptr + ns);
       check_launch("scan_tiles");
-      scan_apply<<<tiles, kScanBlock, 0, s>>>(counts.ptr, ns, tile_sums.ptr, slot_start.ptr, cursor.ptr,
-                                                     0u);
+      scan_apply<<<tiles, kScanBlock, 0, s>>>(counts.ptr, ns, seg.group_log, tile_sums.ptr, slot_start.ptr, cursor.ptr,
+                                              sorted.ptr);
       check_launch("scan_apply");
       break;
     }
@@ -315,7 +398,7 @@ void MsmPlan::stage(int which, const uint32_t* bases, const uint32_t* scalars, c
       if (ranked_sort()) {
         const dim3 grid((unsigned)grid_for(points(), b256), windows);
         msm_place<<<grid, b256, 0, s>>>(digits.as<uint16_t>(), ranks.ptr, points(), half, fixed_base, glv ? 1 : 0,
-                                        slot_start.ptr, sorted.ptr);
+                                        slot_start.ptr, seg.group_log, sorted.ptr);
         check_launch("msm_place");
         break;
       }
@@ -327,35 +410,44 @@ void MsmPlan::stage(int which, const uint32_t* bases, const uint32_t* scalars, c
       // GLV: points run_n..2 run_n - 1 are the phi(P_i) of glv_bases
       const uint32_t* bases2 = glv ? glv_bases.ptr : bases;
       const uint32_t split = glv ? (uint32_t)run_n : 0xffffffffu;
+      if (seg.group_log) {
+        using A = typename std::conditional<std::is_same<F, Fq>::value, Fq, typename PairedOf<F>::type>::type;
+        affine_stage<A>(bases, bases2, split, s);
+        msm_accumulate<A><<<grid_for(seg.heads, 128), 128, 0, s>>>(
+            affine_sums.ptr, affine_sums.ptr, 0xffffffffu, nullptr, slot_start.ptr, (uint32_t)active_slots(), seg.seg_len,
+            buckets.ptr, heads[0].ptr, head_keys[0].ptr);
+        check_launch("msm_accumulate");
+        break;
+      }
       if ((acc_variant == 5 || acc_variant == 6) && std::is_same<F, Fq>::value) {
         // G1 with the accumulator in shared memory, four blocks per SM
         const size_t acc_smem = f64_acc_smem<f64::FqD>(true);
         if (acc_variant == 5)
-          msm_accumulate_f64<f64::FqD, false, true><<<grid_for(heads_max, 128), 128, acc_smem, s>>>(
-              bases, bases2, split, sorted.ptr, slot_start.ptr, (uint32_t)active_slots(), seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
+          msm_accumulate_f64<f64::FqD, false, true><<<grid_for(seg.heads, 128), 128, acc_smem, s>>>(
+              bases, bases2, split, sorted.ptr, slot_start.ptr, (uint32_t)active_slots(), seg.seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
         else
-          msm_accumulate_f64<f64::FqD, true, true><<<grid_for(heads_max, 128), 128, acc_smem, s>>>(
-              bases, bases2, split, sorted.ptr, slot_start.ptr, (uint32_t)active_slots(), seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
+          msm_accumulate_f64<f64::FqD, true, true><<<grid_for(seg.heads, 128), 128, acc_smem, s>>>(
+              bases, bases2, split, sorted.ptr, slot_start.ptr, (uint32_t)active_slots(), seg.seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
       } else if (acc_variant == 3 || (acc_variant > 3 && std::is_same<F, Fq2>::value)) {
         using E = typename std::conditional<std::is_same<F, Fq>::value, f64::FqD, f64::Fq2D>::type;
         const size_t acc_smem = f64_acc_smem<E>();
         if (acc_variant == 3 || acc_variant == 6)
-          msm_accumulate_f64<E, true><<<grid_for(heads_max, 128), 128, acc_smem, s>>>(
-              bases, bases2, split, sorted.ptr, slot_start.ptr, (uint32_t)active_slots(), seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
+          msm_accumulate_f64<E, true><<<grid_for(seg.heads, 128), 128, acc_smem, s>>>(
+              bases, bases2, split, sorted.ptr, slot_start.ptr, (uint32_t)active_slots(), seg.seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
         else
-          msm_accumulate_f64<E, false><<<grid_for(heads_max, 128), 128, acc_smem, s>>>(
-              bases, bases2, split, sorted.ptr, slot_start.ptr, (uint32_t)active_slots(), seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
+          msm_accumulate_f64<E, false><<<grid_for(seg.heads, 128), 128, acc_smem, s>>>(
+              bases, bases2, split, sorted.ptr, slot_start.ptr, (uint32_t)active_slots(), seg.seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
       }
       else if (acc_variant == 1)
-        msm_accumulate<typename CompactOf<F>::type><<<grid_for(heads_max, 128), 128, 0, s>>>(
-            bases, bases2, split, sorted.ptr, slot_start.ptr, (uint32_t)active_slots(), seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
+        msm_accumulate<typename CompactOf<F>::type><<<grid_for(seg.heads, 128), 128, 0, s>>>(
+            bases, bases2, split, sorted.ptr, slot_start.ptr, (uint32_t)active_slots(), seg.seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
       else if (acc_variant == 2)
-        msm_accumulate<typename PairedOf<F>::type><<<grid_for(heads_max, 128), 128, 0, s>>>(
-            bases, bases2, split, sorted.ptr, slot_start.ptr, (uint32_t)active_slots(), seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
+        msm_accumulate<typename PairedOf<F>::type><<<grid_for(seg.heads, 128), 128, 0, s>>>(
+            bases, bases2, split, sorted.ptr, slot_start.ptr, (uint32_t)active_slots(), seg.seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
       else
-        msm_accumulate<F><<<grid_for(heads_max, 128), 128, 0, s>>>(bases, bases2, split, sorted.ptr, slot_start.ptr,
+        msm_accumulate<F><<<grid_for(seg.heads, 128), 128, 0, s>>>(bases, bases2, split, sorted.ptr, slot_start.ptr,
                                                                    (uint32_t)active_slots(),
-                                                                   seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
+                                                                   seg.seg_len, buckets.ptr, heads[0].ptr, head_keys[0].ptr);
       check_launch("msm_accumulate");
       break;
     }
@@ -384,6 +476,46 @@ void MsmPlan::stage(int which, const uint32_t* bases, const uint32_t* scalars, c
   }
 }
 
+// The affine rounds over the run's groups, batch by batch. Batches go to the run's stream and to `side` in turn, so
+// that one's reads and inversions meet the other's products: accumulation at 2^24 36.7 ms in one
+// stream, 33.7 in two, 2^20 2.52 and 2.43; G2 2^20 7.03 and 6.94.
+template <class F>
+void MsmPlan::affine_stage(const uint32_t* bases, const uint32_t* bases2, uint32_t split, cudaStream_t s) {
+  const uint32_t aw = (uint32_t)affine_words();
+  check_cuda(cudaEventRecord(side.fork, s), "fork");
+  check_cuda(cudaStreamWaitEvent(side.stream, side.fork, 0), "fork");
+  const uint32_t log = rounds.group_log, batches = (uint32_t)((rounds.groups + batch_groups - 1) / batch_groups);
+  for (uint32_t b = 0; b < batches; b++) {
+    const AffineLane& lane = affine_lane[b & 1];
+    const cudaStream_t st = (b & 1) ? side.stream : s;
+    auto between = [&](uint32_t k) {  // lane.mid[k]: x of its points, then y
+      const size_t points = (size_t)batch_groups << (log - 1 - k);
+      return PointArray{lane.mid[k].ptr, lane.mid[k].ptr + points * (aw / 2), aw / 2};
+    };
+    for (uint32_t r = 1; r <= log; r++) {
+      const uint32_t pairs_log = log - r;
+      const size_t pairs = (size_t)batch_groups << pairs_log;  // at most
+      const uint32_t per_thread = affine_per_thread(pairs, group, ctx->sm_count);
+      const unsigned blocks = grid_for((pairs + per_thread - 1) / per_thread, kAffineThreads);
+      const PointArray out = r == log ? PointArray{affine_sums.ptr, affine_sums.ptr + aw / 2, aw} : between((r - 1) & 1);
+      const PointArray in = r == 1 ? out : between(r & 1);
+      const AffineRound<F> a{bases, bases2, split, sorted.ptr, in, out, slot_start.ptr, (uint32_t)active_slots(), b, batches,
+                             log, pairs_log, blocks * kAffineThreads, lane.inverses.ptr};
+      const size_t smem = 5 * kAffineThreads * sizeof(F);
+      if (r == 1) msm_affine_prefixes<F, true><<<blocks, kAffineThreads, 0, st>>>(a);
+      else msm_affine_prefixes<F, false><<<blocks, kAffineThreads, 0, st>>>(a);
+      check_launch("msm_affine_prefixes");
+      msm_affine_invert<F><<<grid_for(blocks, kInvertEach), kAffineThreads, 2 * kAffineThreads * sizeof(F), st>>>(a);
+      check_launch("msm_affine_invert");
+      if (r == 1) msm_affine_sums<F, true><<<blocks, kAffineThreads, smem, st>>>(a);
+      else msm_affine_sums<F, false><<<blocks, kAffineThreads, smem, st>>>(a);
+      check_launch("msm_affine_sums");
+    }
+  }
+  check_cuda(cudaEventRecord(side.join, side.stream), "join");
+  check_cuda(cudaStreamWaitEvent(s, side.join, 0), "join");
+}
+
 template <class FC>
 void MsmPlan::tail_stage(int which, cudaStream_t s) {
   switch (which) {
@@ -393,12 +525,13 @@ void MsmPlan::tail_stage(int which, cudaStream_t s) {
       // same or better from 2^18 to 2^24, where threads do more of them per second
       constexpr uint32_t tile = MergeTile<FC>::value;
       const size_t smem = (size_t)tile * (sizeof(Xyzz<FC>) + 12);
-      size_t len = heads_max;  // the largest a level can be (the entry count is on the device)
-      for (uint32_t l = 0; l < merge_levels; l++) {
+      const Segments& seg = segments();
+      size_t len = seg.heads;  // the largest a level can be (the entry count is on the device)
+      for (uint32_t l = 0; l < seg.merge_levels; l++) {
         const size_t out_len = (len + tile - 1) / tile;
         const int src = l & 1, dst = src ^ 1;
         const uint32_t few = group == ZKG_G1 ? 32 : 56;
-        msm_merge<FC><<<(unsigned)out_len, kMergeThreads, smem, s>>>(slot_start.ptr, (uint32_t)active_slots(), seg_len, l, few,
+        msm_merge<FC><<<(unsigned)out_len, kMergeThreads, smem, s>>>(slot_start.ptr, (uint32_t)active_slots(), seg.seg_len, l, few,
                                                                     heads[src].ptr, head_keys[src].ptr, heads[dst].ptr,
                                                                     head_keys[dst].ptr, buckets.ptr);
         check_launch("msm_merge");

@@ -10,6 +10,7 @@
 namespace zkg {
 
 uint32_t default_window(size_t n);
+uint32_t auto_seg_len(size_t entries, int group, int sms);  // points per segment, unless the caller chooses
 void upload_bases(zkg_ctx* ctx, const uint32_t* xy, size_t words, bool mont256, zkg_buf* out);
 // out (windows * n points) <- the fixed-base table of n resident bases for window size c: row w
 // holds 2^(c w) P_i (windows = ceil(255 / c)); queued on the context stream.
@@ -34,7 +35,8 @@ struct MsmPlan {
   zkg_ctx* ctx;
   int group;
   size_t n;
-  uint32_t c, windows = 0, half = 0, seg_len = 0;
+  uint32_t c, windows = 0, half = 0;
+  bool affine;  // may have affine rounds (their scratch doubles the plan's or more)
   // Accumulation kernel form: 0 = integer field products inlined, 1 = through one out-of-line
   // product, 2 = out of line, independent products two per call (G2: one reduction per component of
   // an Fq2 product), 3 / 5 / 6 = bucket arithmetic in
@@ -79,14 +81,43 @@ struct MsmPlan {
   size_t points() const { return glv ? 2 * run_n : run_n; }
   size_t active_slots() const { return fixed_base ? half : slots; }
   uint32_t active_windows() const { return fixed_base ? 1u : windows; }
-  size_t slots = 0, heads_max = 0;
-  uint32_t merge_levels = 0, scan_tiles_n = 0;
+  size_t slots = 0;
+  // What the accumulation kernel sums: groups of 2^group_log entries, each of which the affine rounds
+  // (msm_affine.cuh) have made one point, or the entries themselves (group_log = 0); in segments of
+  // seg_len, one partial sum (head) each at most, merged in merge_levels launches. The rounds belong to the plan's own
+  // accumulation form; the scratch holds both layouts, so that switching the form moves nothing.
+  struct Segments {
+    uint32_t group_log = 0, seg_len = 0, merge_levels = 0;
+    size_t groups = 0, heads = 0;
+  };
+  Segments rounds, plain;
+  int own_variant() const { return group == ZKG_G1 ? 4 : 2; }
+  const Segments& segments() const { return rounds.group_log && acc_variant == own_variant() ? rounds : plain; }
+  uint32_t affine_rounds(size_t entries) const;
+  uint32_t batch_groups = 0;  // of a batch of rounds, at most, which bounds their scratch
+  uint32_t scan_tiles_n = 0;
   ReduceLevels levels;
   std::vector<uint32_t> level_m;
 
   DeviceArray counts, slot_start, cursor, tile_sums, sorted, buckets;
   DeviceArray ranks, digits;  // the ranked sort's rank (32 bits) and digit (16 bits) per (window, point), window-major
   DeviceArray glv_bases;      // GLV mode: phi(P_0)..phi(P_{n-1})
+  DeviceArray affine_sums;    // the rounds' result, one affine point per group
+  // Batches alternate between the run's stream and `side`, each with its own scratch: a round's
+  // products of denominators, one per thread, and a batch's points between rounds, all x then all y.
+  struct AffineLane {
+    DeviceArray inverses, mid[2];
+  };
+  AffineLane affine_lane[2];
+  struct SideStream {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    ~SideStream() {
+      if (stream) cudaStreamDestroy(stream);
+      if (fork) cudaEventDestroy(fork);
+      if (join) cudaEventDestroy(join);
+    }
+  } side;
   DeviceArray heads[2], head_keys[2];
   uint32_t marg_lo = 0, marg_hi = 0, marg_stride = 0;  // the last level's column and row bits (msm_marginals)
   DeviceArray marginals, bit_sums;
@@ -94,7 +125,7 @@ struct MsmPlan {
   zkg_buf result_handle;
   StageTimer timer;
 
-  MsmPlan(zkg_ctx* ctx, int group, size_t n, uint32_t c, uint32_t item_points);
+  MsmPlan(zkg_ctx* ctx, int group, size_t n, uint32_t c, uint32_t item_points, bool affine = true);
   ~MsmPlan() {
     if (result_handle.last_use) cudaEventDestroy(result_handle.last_use);
     if (result_handle.pending_read) cudaEventDestroy(result_handle.pending_read);
@@ -117,9 +148,12 @@ struct MsmPlan {
   void stage(int which, const uint32_t* bases, const uint32_t* scalars, cudaStream_t s);
   template <class FC>
   void tail_stage(int which, cudaStream_t s);
+  template <class F>
+  void affine_stage(const uint32_t* bases, const uint32_t* bases2, uint32_t split, cudaStream_t s);
   // Windows, slots, segments, merge and reduction levels and their scratch, for the current
   // mode (points() and the scalar width); the result buffer is kept.
   void layout();
+  void layout_rounds(uint32_t group_log);
   uint32_t* combine_out = nullptr;  // where the combination of the pass being queued goes
   bool first_pass = true;
   void begin_pass(size_t off, const uint32_t*& bases, const uint32_t*& scalars);

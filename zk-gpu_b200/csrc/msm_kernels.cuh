@@ -523,9 +523,10 @@ __global__ void msm_rank_glv(const uint32_t* __restrict__ scalars, size_t scalar
 // fixed: every window's digits share the buckets, and the entry names point w * n + i of a
 // fixed-base table (2^(c w) P_i at row w). glv: column i holds half i & 1 of scalar i >> 1
 // (msm_rank_glv), point (i >> 1) + (i & 1) n / 2.
+// slot_start counts groups of 2^group_log places.
 __global__ void msm_place(const uint16_t* __restrict__ digits, const uint32_t* __restrict__ ranks, size_t n,
                           uint32_t half, int fixed, int glv, const uint32_t* __restrict__ slot_start,
-                          uint32_t* __restrict__ sorted) {
+                          uint32_t group_log, uint32_t* __restrict__ sorted) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint32_t w = blockIdx.y;
@@ -534,7 +535,7 @@ __global__ void msm_place(const uint16_t* __restrict__ digits, const uint32_t* _
   if (digit == kRankZero) return;
   const uint32_t slot = (fixed ? 0u : w * half) + (digit & 0x7fffu);
   const uint32_t point = fixed ? (uint32_t)e : glv ? (uint32_t)((i >> 1) + (i & 1) * (n >> 1)) : (uint32_t)i;
-  sorted[slot_start[slot] + __ldcs(ranks + e)] = point | ((digit & 0x8000u) ? kNegBit : 0u);
+  sorted[(slot_start[slot] << group_log) + __ldcs(ranks + e)] = point | ((digit & 0x8000u) ? kNegBit : 0u);
 }
 
 // Fixed-base table: row w holds 2^(c w) P_i for every base i (affine, Montgomery form, infinity
@@ -558,6 +559,13 @@ __global__ void msm_fixed_base_table(const uint32_t* __restrict__ bases, size_t 
 }
 
 // ------------------------------------------------------------------ scan (3 phases)
+//
+// Over the slots' numbers of groups: a slot of k entries takes ceil(k / 2^group_log) groups of
+// 2^group_log places in the sorted array (group_log = 0 without affine rounds: groups are entries).
+
+__device__ __forceinline__ uint32_t groups_of(uint32_t entries, uint32_t group_log) {
+  return (entries + (1u << group_log) - 1) >> group_log;
+}
 
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* total, uint32_t* warp_sums) {
   unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -585,14 +593,21 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* t
   return before + x - v;
 }
 
+// Also adds the entries themselves into *entries (zkg_msm_last_entries).
 __global__ void __launch_bounds__(kScanBlock) scan_tile_sums(const uint32_t* __restrict__ in, size_t len,
-                                                             uint32_t* __restrict__ tile_sums) {
+                                                             uint32_t group_log, uint32_t* __restrict__ tile_sums,
+                                                             uint32_t* __restrict__ entries) {
   __shared__ uint32_t warp_sums[32];
   size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
-  uint32_t s = 0;
+  uint32_t s = 0, raw = 0;
 #pragma unroll
   for (int k = 0; k < kScanItems; k++)
-    if (base + k < len) s += in[base + k];
+    if (base + k < len) {
+      raw += in[base + k];
+      s += groups_of(in[base + k], group_log);
+    }
+  raw = __reduce_add_sync(0xffffffffu, raw);
+  if ((threadIdx.x & 31) == 0 && raw) atomicAdd(entries, raw);
   uint32_t total;
   block_exclusive_scan(s, &total, warp_sums);
   if (threadIdx.x == 0) tile_sums[blockIdx.x] = total;
@@ -621,11 +636,13 @@ __global__ void __launch_bounds__(kScanBlock) scan_tiles(uint32_t* __restrict__ 
   if (threadIdx.x == 0) *grand = total;
 }
 
-// out[i] = exclusive prefix of in; also writes it plus out2_bias to out2 (the scatter cursor).
+// out[i] = exclusive prefix of the groups; also each slot's first place to out2 (the scatter cursor),
+// and kPadEntry to the places of its last group that its entries leave free.
 __global__ void __launch_bounds__(kScanBlock) scan_apply(const uint32_t* __restrict__ in, size_t len,
+                                                         uint32_t group_log,
                                                          const uint32_t* __restrict__ tile_offsets,
                                                          uint32_t* __restrict__ out, uint32_t* __restrict__ out2,
-                                                         uint32_t out2_bias) {
+                                                         uint32_t* __restrict__ sorted) {
   __shared__ uint32_t warp_sums[32];
   size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
   uint32_t v[kScanItems];
@@ -633,17 +650,19 @@ __global__ void __launch_bounds__(kScanBlock) scan_apply(const uint32_t* __restr
 #pragma unroll
   for (int k = 0; k < kScanItems; k++) {
     v[k] = base + k < len ? in[base + k] : 0;
-    s += v[k];
+    s += groups_of(v[k], group_log);
   }
   uint32_t total;
   uint32_t run = block_exclusive_scan(s, &total, warp_sums) + tile_offsets[blockIdx.x];
 #pragma unroll
   for (int k = 0; k < kScanItems; k++) {
+    const uint32_t next = run + groups_of(v[k], group_log);
     if (base + k < len) {
       out[base + k] = run;
-      out2[base + k] = run + out2_bias;
+      out2[base + k] = run << group_log;
+      for (uint32_t e = (run << group_log) + v[k]; e < (next << group_log); e++) sorted[e] = kPadEntry;
     }
-    run += v[k];
+    run = next;
   }
 }
 
@@ -669,7 +688,8 @@ __device__ __forceinline__ Affine<F> load_signed_base(const uint32_t* __restrict
 // One thread per segment [t*L, t*L + L) of the sorted entries (all windows concatenated, slot
 // order). slot_start has num_slots + 1 entries; slot_start[num_slots] = total entries.
 // Points below `split` come from `bases`, the others from bases2 (point - split): the GLV
-// entries' P_i and phi(P_i); plain plans pass split = 2^32 - 1.
+// entries' P_i and phi(P_i); plain plans pass split = 2^32 - 1. sorted = null: entry p is point p
+// (the groups' sums that the affine rounds left, slot_start counting groups).
 template <class F>
 __global__ void __launch_bounds__(128) msm_accumulate(const uint32_t* __restrict__ bases,
                                                       const uint32_t* __restrict__ bases2, uint32_t split,
@@ -707,12 +727,13 @@ __global__ void __launch_bounds__(128) msm_accumulate(const uint32_t* __restrict
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa + 16 * k), "l"(g + k) : "memory");
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  uint32_t entry = __ldg(&sorted[p0]);
+  auto entry_at = [&](uint32_t p) { return sorted ? __ldg(&sorted[p]) : p; };
+  uint32_t entry = entry_at(p0);
   uint32_t cur_entry = entry, slot = 0;
   stage_base(0, entry);
   for (uint32_t p = p0; p < p1; p++) {
     if (p + 1 < p1) {
-      entry = __ldg(&sorted[p + 1]);
+      entry = entry_at(p + 1);
       stage_base(slot ^ 1, entry);
       asm volatile("cp.async.wait_group 1;" ::: "memory");  // this point's copy has landed
     } else {

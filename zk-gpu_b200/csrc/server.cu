@@ -109,8 +109,12 @@ const ServerKey* Server::key_for(uint32_t log_m) const {
   return best;
 }
 
+// Whether slots of a size have affine rounds, whose scratch makes a slot of 2^20 points three times as
+// large: where the budget holds twice the slots that may be busy at once, so that no fewer fit.
+bool Server::with_rounds(uint32_t log_m) const { return estimate_bytes(log_m, true) <= budget / (2 * cfg.lanes); }
+
 // Device bytes of a slot, from the same formulas the plans allocate with.
-size_t Server::estimate_bytes(uint32_t log_m) const {
+size_t Server::estimate_bytes(uint32_t log_m, bool rounds) const {
   const size_t m = (size_t)1 << log_m, N = 2 * m;
   auto msm = [&](size_t xw) {
     const uint32_t c = default_window(m), W = (255 + c - 1) / c;
@@ -118,12 +122,17 @@ size_t Server::estimate_bytes(uint32_t log_m) const {
     const uint32_t Wg = (128 + c - 1) / c;
     const size_t B = (size_t)1 << (c - 1), S = (size_t)W * B;
     // (point, window) entries: the GLV plan has Wg windows over 2m points
-    const size_t entries = std::max((size_t)W * m, glv ? (size_t)Wg * 2 * m : 0), L = 8;  // worst-case segment
-    const size_t heads = entries / L + 1;
+    const size_t entries = std::max((size_t)W * m, glv ? (size_t)Wg * 2 * m : 0);
+    const size_t fewest = glv ? (size_t)Wg * 2 * m : entries;
+    const size_t heads = entries / auto_seg_len(fewest, xw == 32 ? ZKG_G1 : ZKG_G2, ctx->sm_count) + 1;
+    // affine rounds: a point per four entries, and two batches' points between rounds
+    const size_t affine = !rounds || entries < (1u << 22)
+                              ? 0
+                              : xw / 2 * (entries / 4 + 2 * S + std::min(entries / 2, (size_t)1 << 25) * 3 / 2);
     // counts, slot starts, cursors; sorted entries, ranks and digits; buckets; heads; running
     // sums; the GLV bases (phi of the m points)
     return 4 * (3 * S + entries * 5 / 2 + S * xw + (heads + heads / 16 + 2) * (xw + 1) + 8 * W * B / 16 * xw / 8 +
-                (glv ? m * 16 : 0) + 4096);
+                (glv ? m * 16 : 0) + affine + 4096);
   };
   // scratch and pass twiddle tables (both directions: 64 bytes per element for the first pass, an
   // eighth of that at most for the later passes' small tables at these sizes)
@@ -142,8 +151,8 @@ std::unique_ptr<ServerSlot> Server::make_slot(uint32_t log_m) {
   const size_t m = (size_t)1 << log_m, N = 2 * m;
   size_t free0 = 0, free1 = 0, total = 0;
   check_cuda(cudaMemGetInfo(&free0, &total), "cudaMemGetInfo");
-  s->g1.reset(new MsmPlan(ctx, ZKG_G1, m, default_window(m), 0));
-  s->g2.reset(new MsmPlan(ctx, ZKG_G2, m, default_window(m), 0));
+  s->g1.reset(new MsmPlan(ctx, ZKG_G1, m, default_window(m), 0, with_rounds(log_m)));
+  s->g2.reset(new MsmPlan(ctx, ZKG_G2, m, default_window(m), 0, with_rounds(log_m)));
   s->ntt.reset(new NttPlan(ctx, log_m + 1));
   s->shift.reset(new CosetShift(ctx, log_m + 1, cfg.coset_g));
   // 1/g as plain words for the unshift

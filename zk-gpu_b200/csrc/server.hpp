@@ -90,7 +90,9 @@ struct Server {
   void dispatcher();
   void builder();
   std::unique_ptr<ServerSlot> make_slot(uint32_t log_m);
-  size_t estimate_bytes(uint32_t log_m) const;
+  bool with_rounds(uint32_t log_m) const;
+  size_t estimate_bytes(uint32_t log_m, bool rounds) const;
+  size_t estimate_bytes(uint32_t log_m) const { return estimate_bytes(log_m, with_rounds(log_m)); }
   const ServerKey* key_for(uint32_t log_m) const;
   void enqueue_work(ServerSlot* s, cudaStream_t main, cudaStream_t b0, cudaStream_t b1);
   void launch(ServerRequest* r, ServerSlot* s);
