@@ -2,32 +2,33 @@
 // level run on different lanes at once, so an operation takes its levels' latency (doubling 3,
 // addition 4) instead of its products' (9 and 14).
 //
-// A group is eight roles, of one lane each for Fq and two for Fq2 (kLanes = 8 or 16 lanes; a warp
-// holds 4 or 2 groups). In Fq2 the two lanes of a role compute one component of a product each, a0 b0
-// - a1 b1 and a0 b1 + a1 b0 through one reduction, and exchange them. Values pass between roles by
-// shuffles within the group; every lane of a warp takes part in every call.
+// A group is eight roles, of one lane each for Fq and two or four for Fq2 (kLanes = 8, 16 or 32 lanes; a
+// warp holds 4, 2 or 1 groups). In Fq2 the two lanes of a role compute one component of a product each,
+// a0 b0 - a1 b1 and a0 b1 + a1 b0 through one reduction, and exchange them; with four lanes (SPLIT = 2)
+// each computes one of the four products, for chains with nothing beside them to fill the warp. Values
+// pass between roles by shuffles within the group; every lane of a warp takes part in every call.
 //
-// A lone warp's product takes 414 ns, an Fq2 product 611 ns; measured on B200 per doubling in the
-// chain of the window combination, G1 1.6 us, G2 2.2 us. Every lane used to hold the whole point and
-// to form every level's sums itself through shared memory: 1.9 and 5.4 us.
+// A lone warp's product takes 414 ns, a b - c d 611 ns; measured on B200 per doubling in the chain of
+// the window combination, G1 1.6 us, G2 2.4 us (two lanes a role 2.65). Every lane used to hold the
+// whole point and to form every level's sums itself through shared memory: 1.9 and 5.4 us.
 #pragma once
 #include "curve.cuh"
 
 namespace zkg {
 
-template <class F>
+template <class F, int SPLIT = 1>
 struct LaneGroup;
-template <class P>
-struct LaneGroup<Fp<P>> {
-  static constexpr unsigned kLanes = 8, kComponents = 1;
+template <class P, int SPLIT>
+struct LaneGroup<Fp<P>, SPLIT> {  // a product of Fq is not split
+  static constexpr unsigned kLanes = 8, kComponents = 1, kPerRole = 1;
 };
-template <class B>
-struct LaneGroup<Fq2T<B>> {
-  static constexpr unsigned kLanes = 16, kComponents = 2;
+template <class B, int SPLIT>
+struct LaneGroup<Fq2T<B>, SPLIT> {
+  static constexpr unsigned kLanes = 16 * SPLIT, kComponents = 2, kPerRole = 2 * SPLIT;
 };
-template <class F>
+template <class F, int SPLIT = 1>
 __device__ __forceinline__ unsigned lane_role() {
-  return (threadIdx.x & (LaneGroup<F>::kLanes - 1)) / LaneGroup<F>::kComponents;
+  return (threadIdx.x & (LaneGroup<F, SPLIT>::kLanes - 1)) / LaneGroup<F, SPLIT>::kPerRole;
 }
 template <class F>
 __device__ __forceinline__ unsigned lane_component() {
@@ -35,20 +36,20 @@ __device__ __forceinline__ unsigned lane_component() {
 }
 
 // The value a role of this group holds (role: may differ between lanes).
-template <class F>
+template <int SPLIT = 1, class F>
 __device__ __forceinline__ F lane_from(const F& v, unsigned role) {
   constexpr unsigned W = sizeof(F) / 4;
-  const unsigned src = role * LaneGroup<F>::kComponents + lane_component<F>();
+  const unsigned src = role * LaneGroup<F, SPLIT>::kPerRole;
   F r;
   const uint32_t* a = reinterpret_cast<const uint32_t*>(&v);
   uint32_t* b = reinterpret_cast<uint32_t*>(&r);
 #pragma unroll
-  for (unsigned i = 0; i < W; i++) b[i] = __shfl_sync(0xffffffffu, a[i], src, LaneGroup<F>::kLanes);
+  for (unsigned i = 0; i < W; i++) b[i] = __shfl_sync(0xffffffffu, a[i], src, LaneGroup<F, SPLIT>::kLanes);
   return r;
 }
-template <class F>
+template <class F, int SPLIT = 1>
 __device__ __forceinline__ bool lane_flag(bool v, unsigned role) {
-  return __shfl_sync(0xffffffffu, (int)v, role * LaneGroup<F>::kComponents, LaneGroup<F>::kLanes) != 0;
+  return __shfl_sync(0xffffffffu, (int)v, role * LaneGroup<F, SPLIT>::kPerRole, LaneGroup<F, SPLIT>::kLanes) != 0;
 }
 
 template <class P>
@@ -64,7 +65,7 @@ __device__ __forceinline__ Fq2T<B> lane_select(bool c, const Fq2T<B>& a, const F
 }
 
 // A role's product and square: for Fq2 each lane its component, then both lanes both.
-template <class P>
+template <int SPLIT = 1, class P>
 __device__ __forceinline__ Fp<P> lane_product(const Fp<P>& a, const Fp<P>& b) {
   return mont_mul_prod(a, b);
 }
@@ -80,9 +81,18 @@ __device__ __forceinline__ Fq2T<B> lane_exchange(const B& own) {
   const bool imaginary = threadIdx.x & 1;
   return Fq2T<B>{lane_select(imaginary, other, own), lane_select(imaginary, own, other)};
 }
-template <class B>
+template <int SPLIT = 1, class B>
 __device__ __forceinline__ Fq2T<B> lane_product(const Fq2T<B>& a, const Fq2T<B>& b) {
   const bool imaginary = threadIdx.x & 1;
+  if constexpr (SPLIT == 2) {  // lanes 0, 2: a0 b0, a1 b1; 1, 3: a0 b1, a1 b0
+    const bool second = threadIdx.x & 2;
+    const B own = mont_mul_prod(lane_select(second, a.b, a.a), lane_select(second != imaginary, b.b, b.a));
+    B other;
+#pragma unroll
+    for (int i = 0; i < 8; i++) other.w[i] = __shfl_xor_sync(0xffffffffu, own.w[i], 2);
+    const B difference = lane_select(second, other, own) - lane_select(second, own, other);
+    return lane_exchange(lane_select(imaginary, own + other, difference));
+  }
   return lane_exchange(reduce_once(mont_mul_add_lazy(a.a, lane_select(imaginary, b.b, b.a),
                                                      lane_select(imaginary, a.b, complement(a.b)),
                                                      lane_select(imaginary, b.a, b.b))));
@@ -94,6 +104,12 @@ __device__ __forceinline__ Fq2T<B> lane_square(const Fq2T<B>& a) {  // (a0 + a1)
                                      lane_select(imaginary, a.b, a.a - a.b)));
 }
 
+// A lane's role in a group of SPLIT lanes a component.
+template <int SPLIT>
+struct LaneRole {
+  unsigned role;
+};
+
 // A point held by a group: x and y in every lane, zz and zzz in role 3's alone.
 template <class F>
 struct LanePoint {
@@ -101,20 +117,21 @@ struct LanePoint {
 };
 
 // 2P (dbl-2008-s-1, a = 0), as xyzz_double. Roles 0, 1 and 3 form V = U^2 for themselves, role 2 X^2;
-// then W = U V, S = X V, M^2, ZZ3 = V ZZ; then W Y, M (S - X3), W ZZZ. role: lane_role.
-template <class F>
-__device__ __forceinline__ LanePoint<F> lane_double(const LanePoint<F>& p, unsigned role) {
+// then W = U V, S = X V, M^2, ZZ3 = V ZZ; then W Y, M (S - X3), W ZZZ.
+template <int SPLIT, class F>
+__device__ __forceinline__ LanePoint<F> lane_double(const LanePoint<F>& p, LaneRole<SPLIT> lane) {
+  const unsigned role = lane.role;
   const F u = dbl(p.y);
   const F l1 = lane_square(lane_select(role == 2, p.x, u));
   const F m = dbl(l1) + l1;
-  const F l2 = lane_product(lane_select(role == 0, u, lane_select(role == 1, p.x, lane_select(role == 2, m, p.zz))),
-                            lane_select(role == 2, m, l1));
-  const F ex = lane_from(l2, role == 2 ? 1u : 0u);  // S in role 2, W in role 3
+  const F l2 = lane_product<SPLIT>(lane_select(role == 0, u, lane_select(role == 1, p.x, lane_select(role == 2, m, p.zz))),
+                                   lane_select(role == 2, m, l1));
+  const F ex = lane_from<SPLIT>(l2, role == 2 ? 1u : 0u);  // S in role 2, W in role 3
   const F x3 = l2 - dbl(ex);
-  const F l3 = lane_product(lane_select(role == 2, m, lane_select(role == 3, ex, l2)),
-                            lane_select(role == 2, ex - x3, lane_select(role == 3, p.zzz, p.y)));
-  const F y3 = l3 - lane_from(l3, 0);
-  return LanePoint<F>{lane_from(x3, 2), lane_from(y3, 2), l2, l3};
+  const F l3 = lane_product<SPLIT>(lane_select(role == 2, m, lane_select(role == 3, ex, l2)),
+                                   lane_select(role == 2, ex - x3, lane_select(role == 3, p.zzz, p.y)));
+  const F y3 = l3 - lane_from<SPLIT>(l3, 0);
+  return LanePoint<F>{lane_from<SPLIT>(x3, 2), lane_from<SPLIT>(y3, 2), l2, l3};
 }
 
 // A point of memory in a group's lanes, and back (out: any memory the group may write).
@@ -132,10 +149,10 @@ __device__ __forceinline__ void lane_store_elem(uint32_t* p, const Fq2T<B>& v) {
   const bool imaginary = threadIdx.x & 1;
   store_fe(p + (imaginary ? 8 : 0), lane_select(imaginary, v.b, v.a));
 }
-template <class F>
+template <int SPLIT = 1, class F>
 __device__ __forceinline__ void lane_store(uint32_t* out, const LanePoint<F>& p) {
   constexpr int W = FieldWords<F>::value;
-  if (lane_role<F>() == 3) {
+  if (lane_role<F, SPLIT>() == 3) {
     lane_store_elem(out, p.x);
     lane_store_elem(out + W, p.y);
     lane_store_elem(out + 2 * W, p.zz);
@@ -145,10 +162,10 @@ __device__ __forceinline__ void lane_store(uint32_t* out, const LanePoint<F>& p)
 
 // *out = *p + *q (add-2008-s), as xyzz_add, for points in memory that the group may read; out may be p
 // or q. A group with active = false takes part and writes nothing (p and q: any readable points).
-template <class F>
+template <class F, int SPLIT = 1>
 __device__ __forceinline__ void lane_add(const uint32_t* p, const uint32_t* q, uint32_t* out, bool active) {
   constexpr int W = FieldWords<F>::value;
-  const unsigned role = lane_role<F>();
+  const unsigned role = lane_role<F, SPLIT>();
   // roles 0..5: X1 ZZ2, X2 ZZ1, Y1 ZZZ2, Y2 ZZZ1, ZZ1 ZZ2, ZZZ1 ZZZ2
   const bool second = role == 1 || role == 3;
   const uint32_t* const pa = second ? q : p;
@@ -156,24 +173,25 @@ __device__ __forceinline__ void lane_add(const uint32_t* p, const uint32_t* q, u
   const int ca = role < 2 ? 0 : role < 4 ? 1 : (role & 1) ? 3 : 2;
   const int cb = role < 2 ? 2 : role < 4 ? 3 : ca;
   const F a = load_elem<F>(pa + ca * W), b = load_elem<F>(pb + cb * W);
-  const bool inf_p = lane_flag<F>(a.is_zero(), 4), inf_q = lane_flag<F>(b.is_zero(), 4);
-  const F l1 = lane_product(a, b);
-  const F other = lane_from(l1, role ^ 1);
+  const bool inf_p = lane_flag<F, SPLIT>(a.is_zero(), 4), inf_q = lane_flag<F, SPLIT>(b.is_zero(), 4);
+  const F l1 = lane_product<SPLIT>(a, b);
+  const F other = lane_from<SPLIT>(l1, role ^ 1);
   const F d = lane_select(role & 1, l1 - other, other - l1);  // roles 0, 1: P; 2, 3: R
-  const bool p_zero = lane_flag<F>(d.is_zero(), 0), r_zero = lane_flag<F>(d.is_zero(), 2);
+  const bool p_zero = lane_flag<F, SPLIT>(d.is_zero(), 0), r_zero = lane_flag<F, SPLIT>(d.is_zero(), 2);
   const F sq = lane_square(d);                                  // PP; RR
-  const F l3 = lane_product(lane_select(role == 1, d, l1), lane_from(sq, 0));  // Q, PPP, -, -, ZZ3
-  const F qq = lane_from(l3, 0), ppp = lane_from(l3, 1);
+  const F l3 = lane_product<SPLIT>(lane_select(role == 1, d, l1), lane_from<SPLIT>(sq, 0));  // Q, PPP, -, -, ZZ3
+  const F qq = lane_from<SPLIT>(l3, 0), ppp = lane_from<SPLIT>(l3, 1);
   const F x3 = (sq - ppp) - dbl(qq);
-  const F l4 = lane_product(lane_select(role == 3, d, l1), lane_select(role == 3, qq - x3, ppp));  // 2: S1 PPP, 3: R (Q - X3), 5: ZZZ3
-  const F y3 = l4 - lane_from(l4, 2);
+  // 2: S1 PPP, 3: R (Q - X3), 5: ZZZ3
+  const F l4 = lane_product<SPLIT>(lane_select(role == 3, d, l1), lane_select(role == 3, qq - x3, ppp));
+  const F y3 = l4 - lane_from<SPLIT>(l4, 2);
   __syncwarp();
   if (!active) return;
   if (inf_p || inf_q) {
     const uint32_t* const src = inf_p ? q : p;
     if (src != out && role < 4) lane_store_elem(out + role * W, load_elem<F>(src + role * W));
   } else if (p_zero) {
-    if (role == 0 && lane_component<F>() == 0)
+    if ((threadIdx.x & (LaneGroup<F, SPLIT>::kLanes - 1)) == 0)
       store_xyzz(out, r_zero ? xyzz_double_call(load_xyzz<F>(p)) : xyzz_infinity<F>());
   } else if (role == 3) {
     lane_store_elem(out, x3);

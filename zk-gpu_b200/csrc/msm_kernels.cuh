@@ -1033,14 +1033,14 @@ __global__ void __launch_bounds__(SubsetThreads<F>::value)
 // down, S = 2^chunk_log S + its total.
 constexpr uint32_t kFoldGroups = 4;
 template <class F>
-__global__ void __launch_bounds__(kFoldGroups * LaneGroup<F>::kLanes)
+__global__ void __launch_bounds__(kFoldGroups * LaneGroup<F, 2>::kLanes)
     msm_window_fold(const uint32_t* __restrict__ bits, uint32_t bit_count, const uint32_t* __restrict__ totals,
                     uint32_t totals_stride, uint32_t levels, uint32_t chunk_log, uint32_t* __restrict__ window_sums) {
   constexpr int XW = PointWords<F>::xyzz;
   __shared__ __align__(16) uint32_t share[kFoldGroups][XW];
   __shared__ __align__(16) uint32_t none[XW];  // the point at infinity
-  const uint32_t w = blockIdx.x, group = threadIdx.x / LaneGroup<F>::kLanes;
-  const unsigned role = lane_role<F>();
+  const uint32_t w = blockIdx.x, group = threadIdx.x / LaneGroup<F, 2>::kLanes;
+  const LaneRole<2> role{lane_role<F, 2>()};
   const uint32_t* const z = bits + (size_t)w * (bit_count + 1) * XW;
   const uint32_t per = (bit_count + kFoldGroups - 1) / kFoldGroups, first = group * per;
   for (uint32_t i = threadIdx.x; i < XW; i += blockDim.x) none[i] = 0;
@@ -1050,14 +1050,14 @@ __global__ void __launch_bounds__(kFoldGroups * LaneGroup<F>::kLanes)
   LanePoint<F> acc = lane_load<F>(bit(first + per - 1));
   for (uint32_t k = per - 1; k-- > 0;) {
     acc = lane_double(acc, role);
-    lane_store(mine, acc);
+    lane_store<2>(mine, acc);
     __syncwarp();
-    lane_add<F>(mine, bit(first + k), mine, true);
+    lane_add<F, 2>(mine, bit(first + k), mine, true);
     __syncwarp();
     acc = lane_load<F>(mine);
     __syncwarp();
   }
-  if (per == 1) lane_store(mine, acc);
+  if (per == 1) lane_store<2>(mine, acc);
   __syncthreads();
   if (threadIdx.x >= 32) return;
   const bool lead = group == 0;
@@ -1067,9 +1067,9 @@ __global__ void __launch_bounds__(kFoldGroups * LaneGroup<F>::kLanes)
     for (uint32_t d = 0; d < doublings; d++) v = lane_double(v, role);
     __syncwarp();
     // the sum goes beside what it reads: `none`, which no later step needs
-    if (lead) lane_store(none, v);
+    if (lead) lane_store<2>(none, v);
     __syncwarp();
-    lane_add<F>(none, add, sum, lead);
+    lane_add<F, 2>(none, add, sum, lead);
     __syncwarp();
   };
   LanePoint<F> v = lane_load<F>(sum);
@@ -1094,20 +1094,20 @@ __global__ void __launch_bounds__(32) msm_combine_lanes(const uint32_t* __restri
                                                         uint32_t base, uint32_t extra, uint32_t* __restrict__ result) {
   constexpr int XW = PointWords<F>::xyzz;
   __shared__ __align__(16) uint32_t sum[XW];
-  const bool first = threadIdx.x < LaneGroup<F>::kLanes;
-  const unsigned sm = lane_role<F>();
+  const bool first = threadIdx.x < LaneGroup<F, 2>::kLanes;
+  const LaneRole<2> sm{lane_role<F, 2>()};
   LanePoint<F> acc = lane_load<F>(window_sums + (size_t)(windows - 1) * XW);
   for (int w = (int)windows - 2; w >= 0; w--) {
     const uint32_t width = base + ((uint32_t)w < extra ? 1u : 0u);
     for (uint32_t k = 0; k < width; k++) acc = lane_double(acc, sm);
-    if (first) lane_store(sum, acc);
+    if (first) lane_store<2>(sum, acc);
     __syncwarp();
-    lane_add<F>(sum, window_sums + (size_t)w * XW, sum, first);
+    lane_add<F, 2>(sum, window_sums + (size_t)w * XW, sum, first);
     __syncwarp();
     acc = lane_load<F>(sum);
     __syncwarp();
   }
-  if (first) lane_store(result, acc);
+  if (first) lane_store<2>(result, acc);
 }
 
 // result <- result + partial (XYZZ, one thread): the passes of a run over more points than one
