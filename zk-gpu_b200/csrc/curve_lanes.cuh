@@ -134,6 +134,109 @@ __device__ __forceinline__ LanePoint<F> lane_double(const LanePoint<F>& p, LaneR
   return LanePoint<F>{lane_from<SPLIT>(x3, 2), lane_from<SPLIT>(y3, 2), l2, l3};
 }
 
+// Sums left between p and 2^256 for a product's operand (a p + p stays below 2^256 for a <= 4).
+template <class P>
+__device__ __forceinline__ Fp<P> lane_sum(const Fp<P>& a, const Fp<P>& b) {
+  Fp<P> r;
+  asm("add.cc.u32  %0, %8, %16;\n\t"
+      "addc.cc.u32 %1, %9, %17;\n\t"
+      "addc.cc.u32 %2, %10, %18;\n\t"
+      "addc.cc.u32 %3, %11, %19;\n\t"
+      "addc.cc.u32 %4, %12, %20;\n\t"
+      "addc.cc.u32 %5, %13, %21;\n\t"
+      "addc.cc.u32 %6, %14, %22;\n\t"
+      "addc.u32    %7, %15, %23;"
+      : "=&r"(r.w[0]), "=&r"(r.w[1]), "=&r"(r.w[2]), "=&r"(r.w[3]), "=&r"(r.w[4]), "=&r"(r.w[5]), "=&r"(r.w[6]),
+        "=&r"(r.w[7])
+      : "r"(a.w[0]), "r"(a.w[1]), "r"(a.w[2]), "r"(a.w[3]), "r"(a.w[4]), "r"(a.w[5]), "r"(a.w[6]), "r"(a.w[7]),
+        "r"(b.w[0]), "r"(b.w[1]), "r"(b.w[2]), "r"(b.w[3]), "r"(b.w[4]), "r"(b.w[5]), "r"(b.w[6]), "r"(b.w[7]));
+  return r;
+}
+template <int BITS, class P>
+__device__ __forceinline__ Fp<P> lane_shift(const Fp<P>& a) {  // 2^BITS a
+  Fp<P> r;
+  r.w[0] = a.w[0] << BITS;
+#pragma unroll
+  for (int i = 1; i < 8; i++) r.w[i] = __funnelshift_l(a.w[i - 1], a.w[i], BITS);
+  return r;
+}
+template <class P>
+__device__ __forceinline__ Fp<P> lane_complement(const Fp<P>& a) {
+  return complement(a);
+}
+template <class P>
+__device__ __forceinline__ Fp<P> lane_halve(const Fp<P>& a) {
+  constexpr uint32_t q[8] = {P::P0, P::P1, P::P2, P::P3, P::P4, P::P5, P::P6, P::P7};
+  Fp<P> p, r;
+#pragma unroll
+  for (int i = 0; i < 8; i++) p.w[i] = (a.w[0] & 1) ? q[i] : 0;
+  const Fp<P> s = lane_sum(a, p);
+#pragma unroll
+  for (int i = 0; i < 7; i++) r.w[i] = __funnelshift_r(s.w[i], s.w[i + 1], 1);
+  r.w[7] = s.w[7] >> 1;
+  return r;
+}
+template <class B>
+__device__ __forceinline__ Fq2T<B> lane_sum(const Fq2T<B>& a, const Fq2T<B>& b) {
+  return Fq2T<B>{lane_sum(a.a, b.a), lane_sum(a.b, b.b)};
+}
+template <int BITS, class B>
+__device__ __forceinline__ Fq2T<B> lane_shift(const Fq2T<B>& a) {
+  return Fq2T<B>{lane_shift<BITS>(a.a), lane_shift<BITS>(a.b)};
+}
+template <class B>
+__device__ __forceinline__ Fq2T<B> lane_complement(const Fq2T<B>& a) {
+  return Fq2T<B>{complement(a.a), complement(a.b)};
+}
+template <class B>
+__device__ __forceinline__ Fq2T<B> lane_halve(const Fq2T<B>& a) {
+  return Fq2T<B>{lane_halve(a.a), lane_halve(a.b)};
+}
+
+// A point through repeated doublings, two products deep each instead of dbl-2008-s-1's three. With
+// D = Y^2 - X^3 (which doubling multiplies by (2Y)^6, whatever curve y^2 = x^3 + b the point is on) and A = Y^2,
+//   X' = X (A - 9D),  Y' = (A + 9D)^2 - 108 D^2,  D' = 64 D A^3,  ZZ' = 4A ZZ,  ZZZ' = 8 Y A ZZZ,
+// the same values. Kept: V = 9D and T = 12D, so that 108 D^2 = V T. A doubling forms A, V, T, 2Y ZZZ/2
+// from the last one's products, then its own, one a role:
+//   0: (A + V)^2   1: V T   2: X'   3: V 4A   4: T 4A   5: A 4A   6: ZZ'   7: ZZZ'/2
+// V' = 4 (V 4A) (A 4A), T' likewise. Operands are left up to 4p, or 2p by 2p: products come out below 2p
+// before their one subtraction.
+template <class F>
+struct LaneChain {
+  F v;  // the role's
+};
+
+template <class F, int SPLIT>
+__device__ __forceinline__ LaneChain<F> lane_chain(const uint32_t* p, LaneRole<SPLIT> lane) {
+  constexpr int W = FieldWords<F>::value;
+  const unsigned role = lane.role;
+  const F x = load_elem<F>(p), y = load_elem<F>(p + W);
+  const F own = load_elem<F>(p + (role == 6 ? 2 : role == 7 ? 3 : role & 1) * W);  // X or Y, ZZ, ZZZ
+  const F sq = lane_square(lane_select(role == 1, y, x));
+  const F d = lane_from<SPLIT>(sq, 1) - lane_product<SPLIT>(lane_from<SPLIT>(sq, 0), x);
+  const F d3 = dbl(d) + d, d6 = dbl(d3);
+  const F quarter = lane_halve(lane_halve(F::one()));  // for role 5: V = 4 (9D) / 4
+  F v = lane_select(role == 0, y, own);
+  v = lane_select(role == 1, F::zero(), lane_select(role == 2, x, v));
+  v = lane_select(role == 3, d6 + d3, lane_select(role == 4, dbl(d6), v));
+  v = lane_select(role == 5, quarter, lane_select(role == 7, lane_halve(own), v));
+  return LaneChain<F>{v};
+}
+template <int SPLIT, class F>
+__device__ __forceinline__ LaneChain<F> lane_double(const LaneChain<F>& c, LaneRole<SPLIT> lane) {
+  const unsigned role = lane.role;
+  const bool vt = role == 1 || role == 3 || role == 4;  // 3: V', 1 and 4: T'; the others: Y'
+  const F s = lane_from<SPLIT>(c.v, vt ? 5u : 0u), t = lane_from<SPLIT>(c.v, !vt ? 1u : role == 3 ? 3u : 4u);
+  const F y = s - t;
+  const F l1 = lane_product<SPLIT>(lane_select(vt, lane_shift<2>(t), y),
+                                   lane_select(vt, s, lane_select(role == 7, lane_shift<1>(c.v), y)));
+  const F a = lane_from<SPLIT>(l1, 0), v = lane_from<SPLIT>(l1, 3);
+  const F sum = lane_sum(a, lane_select(role == 2, lane_complement(v), v));
+  const F left = lane_select(role == 0 || role == 2, sum, lane_select(role == 1, v, lane_shift<2>(a)));
+  const F kept = lane_select(role == 2 || role == 6, c.v, l1);  // X, ZZ; T, V, 2Y ZZZ/2; A in role 5
+  return LaneChain<F>{lane_product<SPLIT>(left, lane_select(role == 0, sum, kept))};
+}
+
 // A point of memory in a group's lanes, and back (out: any memory the group may write).
 template <class F>
 __device__ __forceinline__ LanePoint<F> lane_load(const uint32_t* p) {
@@ -158,6 +261,18 @@ __device__ __forceinline__ void lane_store(uint32_t* out, const LanePoint<F>& p)
     lane_store_elem(out + 2 * W, p.zz);
     lane_store_elem(out + 3 * W, p.zzz);
   }
+}
+
+template <int SPLIT, class F>
+__device__ __forceinline__ void lane_store(uint32_t* out, const LaneChain<F>& c, bool active) {
+  constexpr int W = FieldWords<F>::value;
+  const unsigned role = lane_role<F, SPLIT>();
+  const F y = c.v - lane_from<SPLIT>(c.v, 1);  // in role 0
+  if (!active) return;
+  if (role == 0) lane_store_elem(out + W, y);
+  if (role == 2) lane_store_elem(out, c.v);
+  if (role == 6) lane_store_elem(out + 2 * W, c.v);
+  if (role == 7) lane_store_elem(out + 3 * W, dbl(c.v));
 }
 
 // *out = *p + *q (add-2008-s), as xyzz_add, for points in memory that the group may read; out may be p

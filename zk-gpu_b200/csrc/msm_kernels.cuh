@@ -1062,26 +1062,19 @@ __global__ void __launch_bounds__(kFoldGroups * LaneGroup<F, 2>::kLanes)
   if (threadIdx.x >= 32) return;
   const bool lead = group == 0;
   uint32_t* const sum = share[kFoldGroups - 1];  // starts as the top share
-  auto fold = [&](const LanePoint<F>& start, uint32_t doublings, const uint32_t* add) {  // into sum
-    LanePoint<F> v = start;
+  auto fold = [&](uint32_t doublings, const uint32_t* add) {  // sum <- 2^doublings sum + add
+    LaneChain<F> v = lane_chain<F>(sum, role);
     for (uint32_t d = 0; d < doublings; d++) v = lane_double(v, role);
     __syncwarp();
-    // the sum goes beside what it reads: `none`, which no later step needs
-    if (lead) lane_store<2>(none, v);
+    lane_store<2>(none, v, lead);  // beside what it reads; no later step needs the point at infinity
     __syncwarp();
     lane_add<F, 2>(none, add, sum, lead);
     __syncwarp();
   };
-  LanePoint<F> v = lane_load<F>(sum);
-  for (uint32_t g = kFoldGroups - 1; g-- > 0;) {
-    fold(v, per, share[g]);
-    v = lane_load<F>(sum);
-  }
-  fold(v, 0, z + (size_t)bit_count * XW);
-  for (uint32_t l = levels; l-- > 0;) {
-    v = lane_load<F>(sum);
-    fold(v, chunk_log, totals + ((size_t)w * totals_stride + l) * XW);
-  }
+  for (uint32_t g = kFoldGroups - 1; g-- > 0;) fold(per, share[g]);
+  lane_add<F, 2>(sum, z + (size_t)bit_count * XW, sum, lead);
+  __syncwarp();
+  for (uint32_t l = levels; l-- > 0;) fold(chunk_log, totals + ((size_t)w * totals_stride + l) * XW);
   for (uint32_t i = threadIdx.x; i < XW; i += 32) window_sums[(size_t)w * XW + i] = sum[i];
 }
 
@@ -1096,18 +1089,19 @@ __global__ void __launch_bounds__(32) msm_combine_lanes(const uint32_t* __restri
   __shared__ __align__(16) uint32_t sum[XW];
   const bool first = threadIdx.x < LaneGroup<F, 2>::kLanes;
   const LaneRole<2> sm{lane_role<F, 2>()};
-  LanePoint<F> acc = lane_load<F>(window_sums + (size_t)(windows - 1) * XW);
+  const uint32_t* top = window_sums + (size_t)(windows - 1) * XW;
   for (int w = (int)windows - 2; w >= 0; w--) {
     const uint32_t width = base + ((uint32_t)w < extra ? 1u : 0u);
+    LaneChain<F> acc = lane_chain<F>(top, sm);
     for (uint32_t k = 0; k < width; k++) acc = lane_double(acc, sm);
-    if (first) lane_store<2>(sum, acc);
+    __syncwarp();
+    lane_store<2>(sum, acc, first);
     __syncwarp();
     lane_add<F, 2>(sum, window_sums + (size_t)w * XW, sum, first);
     __syncwarp();
-    acc = lane_load<F>(sum);
-    __syncwarp();
+    top = sum;
   }
-  if (first) lane_store<2>(result, acc);
+  for (uint32_t i = threadIdx.x; i < XW; i += 32) result[i] = top[i];
 }
 
 // result <- result + partial (XYZZ, one thread): the passes of a run over more points than one
