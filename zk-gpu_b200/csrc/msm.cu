@@ -452,15 +452,13 @@ void MsmPlan::stage(int which, const uint32_t* bases, const uint32_t* scalars, c
       break;
     }
     case kStageCombine:
-      // c (W - 1) dependent doublings: one group of lanes, each level's independent products on
-      // separate lanes (curve_lanes.cuh).
-      if constexpr (std::is_same<F, Fq>::value)
-        msm_combine_lanes<Fq><<<1, 32, 0, s>>>(window_sums.ptr, active_windows(), glv ? 128u / windows : c,
-                                               glv ? 128u % windows : 0u, combine_out);
-      else
-        msm_combine_lanes<typename CompactOf<F>::type><<<1, 32, 0, s>>>(window_sums.ptr, active_windows(),
-                                                                         glv ? 128u / windows : c,
-                                                                         glv ? 128u % windows : 0u, combine_out);
+      {
+        // a warp for each pair of windows (msm_combine_lanes)
+        using A = typename std::conditional<std::is_same<F, Fq>::value, Fq, typename CompactOf<F>::type>::type;
+        const uint32_t width = glv ? 128u / windows : c, extra = glv ? 128u % windows : 0u;
+        msm_combine_lanes<A><<<1, 32 * std::max(1u, active_windows() / 2), 0, s>>>(window_sums.ptr, active_windows(), width,
+                                                                                    extra, combine_out);
+      }
       check_launch("msm_combine_lanes");
       if (!first_pass) {  // a later pass: add its point into the result
         msm_add_partial<F><<<1, 32, 0, s>>>(result.ptr, partial.ptr);

@@ -1078,30 +1078,38 @@ __global__ void __launch_bounds__(kFoldGroups * LaneGroup<F, 2>::kLanes)
   for (uint32_t i = threadIdx.x; i < XW; i += 32) window_sums[(size_t)w * XW + i] = sum[i];
 }
 
-// result = sum_w 2^(pos_w) S_w by Horner from the top window (msm_combine.wgsl:13-22), by one group
-// of lanes (curve_lanes.cuh; the warp's other groups repeat its work). Window w is `base` bits wide,
-// or base + 1 for w < extra (pos_w is the sum of the widths below w): base = c, extra = 0 for the
-// plain windows, the glv_window_width split for GLV. Bound by the latency of the doublings' products.
+// result = sum_w 2^(pos_w) S_w (msm_combine.wgsl:13-22), one group of lanes (curve_lanes.cuh) a warp; a warp's
+// other groups repeat its work. Window w is `base` bits wide, or base + 1 for w < extra (pos_w is the
+// sum of the widths below w): base = c, extra = 0 for the plain windows, the glv_window_width split for
+// GLV. Neighbours meet pairwise, 2, 4, 8 .. windows at a time counted from the top one: the top
+// windows' doublings are the chain that any order has, but only log2 W additions lie on it. Bound by
+// the latency of the doublings' products; one chain (Horner) took W - 1 additions, 5.7 us each with
+// their start of a chain (G2 8.9): G1 of 12 windows 0.169 ms, now 0.155, G2 of 24 0.495, now 0.440.
+constexpr uint32_t kCombineWindows = 32;  // 255 bits in windows of 9, at most
 template <class F>
-__global__ void __launch_bounds__(32) msm_combine_lanes(const uint32_t* __restrict__ window_sums, uint32_t windows,
-                                                        uint32_t base, uint32_t extra, uint32_t* __restrict__ result) {
+__global__ void __launch_bounds__(kCombineWindows / 2 * 32)
+    msm_combine_lanes(const uint32_t* __restrict__ window_sums, uint32_t windows, uint32_t base, uint32_t extra,
+                      uint32_t* __restrict__ result) {
   constexpr int XW = PointWords<F>::xyzz;
-  __shared__ __align__(16) uint32_t sum[XW];
-  const bool first = threadIdx.x < LaneGroup<F, 2>::kLanes;
+  __shared__ __align__(16) uint32_t part[kCombineWindows][XW];  // from the top window down
+  const bool first = (threadIdx.x & 31) < LaneGroup<F, 2>::kLanes;
   const LaneRole<2> sm{lane_role<F, 2>()};
-  const uint32_t* top = window_sums + (size_t)(windows - 1) * XW;
-  for (int w = (int)windows - 2; w >= 0; w--) {
-    const uint32_t width = base + ((uint32_t)w < extra ? 1u : 0u);
-    LaneChain<F> acc = lane_chain<F>(top, sm);
+  auto pos = [&](uint32_t w) { return w * base + min(w, extra); };
+  for (uint32_t i = threadIdx.x; i < windows * XW; i += blockDim.x) part[windows - 1 - i / XW][i % XW] = window_sums[i];
+  for (uint32_t span = 1; span < windows; span <<= 1) {
+    __syncthreads();
+    const uint32_t high = threadIdx.x / 32 * 2 * span, low = high + span;  // this warp's pair
+    if (low >= windows) continue;
+    const uint32_t width = pos(windows - low) - pos(windows - min(low + span, windows));  // of the low part
+    LaneChain<F> acc = lane_chain<F>(part[high], sm);
     for (uint32_t k = 0; k < width; k++) acc = lane_double(acc, sm);
     __syncwarp();
-    lane_store<2>(sum, acc, first);
+    lane_store<2>(part[high], acc, first);
     __syncwarp();
-    lane_add<F, 2>(sum, window_sums + (size_t)w * XW, sum, first);
-    __syncwarp();
-    top = sum;
+    lane_add<F, 2>(part[high], part[low], part[high], first);
   }
-  for (uint32_t i = threadIdx.x; i < XW; i += 32) result[i] = top[i];
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < XW; i += blockDim.x) result[i] = part[0][i];
 }
 
 // result <- result + partial (XYZZ, one thread): the passes of a run over more points than one
