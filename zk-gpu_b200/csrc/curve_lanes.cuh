@@ -1,5 +1,5 @@
 // XYZZ doubling and addition by a group of lanes: the independent field products of each dependency
-// level run on different lanes at once, so an operation takes its levels' latency (doubling 3,
+// level run on different lanes at once, so an operation takes its levels' latency (doubling 2,
 // addition 4) instead of its products' (9 and 14).
 //
 // A group is eight roles, of one lane each for Fq and two or four for Fq2 (kLanes = 8, 16 or 32 lanes; a
@@ -111,30 +111,6 @@ struct LaneRole {
   unsigned role;
 };
 
-// A point held by a group: x and y in every lane, zz and zzz in role 3's alone.
-template <class F>
-struct LanePoint {
-  F x, y, zz, zzz;
-};
-
-// 2P (dbl-2008-s-1, a = 0), as xyzz_double. Roles 0, 1 and 3 form V = U^2 for themselves, role 2 X^2;
-// then W = U V, S = X V, M^2, ZZ3 = V ZZ; then W Y, M (S - X3), W ZZZ.
-template <int SPLIT, class F>
-__device__ __forceinline__ LanePoint<F> lane_double(const LanePoint<F>& p, LaneRole<SPLIT> lane) {
-  const unsigned role = lane.role;
-  const F u = dbl(p.y);
-  const F l1 = lane_square(lane_select(role == 2, p.x, u));
-  const F m = dbl(l1) + l1;
-  const F l2 = lane_product<SPLIT>(lane_select(role == 0, u, lane_select(role == 1, p.x, lane_select(role == 2, m, p.zz))),
-                                   lane_select(role == 2, m, l1));
-  const F ex = lane_from<SPLIT>(l2, role == 2 ? 1u : 0u);  // S in role 2, W in role 3
-  const F x3 = l2 - dbl(ex);
-  const F l3 = lane_product<SPLIT>(lane_select(role == 2, m, lane_select(role == 3, ex, l2)),
-                                   lane_select(role == 2, ex - x3, lane_select(role == 3, p.zzz, p.y)));
-  const F y3 = l3 - lane_from<SPLIT>(l3, 0);
-  return LanePoint<F>{lane_from<SPLIT>(x3, 2), lane_from<SPLIT>(y3, 2), l2, l3};
-}
-
 // Sums left between p and 2^256 for a product's operand (a p + p stays below 2^256 for a <= 4).
 template <class P>
 __device__ __forceinline__ Fp<P> lane_sum(const Fp<P>& a, const Fp<P>& b) {
@@ -238,12 +214,7 @@ __device__ __forceinline__ LaneChain<F> lane_double(const LaneChain<F>& c, LaneR
   return LaneChain<F>{lane_product<SPLIT>(left, lane_select(role == 0, sum, kept))};
 }
 
-// A point of memory in a group's lanes, and back (out: any memory the group may write).
-template <class F>
-__device__ __forceinline__ LanePoint<F> lane_load(const uint32_t* p) {
-  constexpr int W = FieldWords<F>::value;
-  return LanePoint<F>{load_elem<F>(p), load_elem<F>(p + W), load_elem<F>(p + 2 * W), load_elem<F>(p + 3 * W)};
-}
+// A group's values to memory that it may write.
 template <class P>
 __device__ __forceinline__ void lane_store_elem(uint32_t* p, const Fp<P>& v) {
   store_fe(p, v);
@@ -253,17 +224,6 @@ __device__ __forceinline__ void lane_store_elem(uint32_t* p, const Fq2T<B>& v) {
   const bool imaginary = threadIdx.x & 1;
   store_fe(p + (imaginary ? 8 : 0), lane_select(imaginary, v.b, v.a));
 }
-template <int SPLIT = 1, class F>
-__device__ __forceinline__ void lane_store(uint32_t* out, const LanePoint<F>& p) {
-  constexpr int W = FieldWords<F>::value;
-  if (lane_role<F, SPLIT>() == 3) {
-    lane_store_elem(out, p.x);
-    lane_store_elem(out + W, p.y);
-    lane_store_elem(out + 2 * W, p.zz);
-    lane_store_elem(out + 3 * W, p.zzz);
-  }
-}
-
 template <int SPLIT, class F>
 __device__ __forceinline__ void lane_store(uint32_t* out, const LaneChain<F>& c, bool active) {
   constexpr int W = FieldWords<F>::value;

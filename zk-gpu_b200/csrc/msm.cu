@@ -567,7 +567,7 @@ void MsmPlan::tail_stage(int which, cudaStream_t s) {
       msm_bit_sums<FC><<<dim3(marg_lo + marg_hi + 1, active_windows()), threads, 0, s>>>(
           marginals.ptr, marg_stride, m, marg_lo, marg_hi, bit_sums.ptr);
       check_launch("msm_bit_sums");
-      msm_window_fold<FC><<<active_windows(), kFoldGroups * LaneGroup<FC, 2>::kLanes, 0, s>>>(
+      msm_window_fold<FC><<<active_windows(), 32 * std::max(1u, (marg_lo + marg_hi + 1) / 2), 0, s>>>(
           bit_sums.ptr, marg_lo + marg_hi, marginals.ptr + ((size_t)(1u << marg_lo) + rows) * xyzz_words(), marg_stride, l,
           levels.chunk_log, window_sums.ptr);
       check_launch("msm_window_fold");

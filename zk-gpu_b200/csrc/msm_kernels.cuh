@@ -1028,79 +1028,19 @@ __global__ void __launch_bounds__(SubsetThreads<F>::value)
   subset_sum<F>(s, high ? columns + (size_t)cols * XW : columns, nullptr, bits + ((size_t)w * (lo + hi + 1) + k) * XW, sh);
 }
 
-// S_w from the Z_k: kFoldGroups groups of lanes run Horner over a share of the bits each, the first
-// folds the shares and adds the sum of all values; then for each chunked level, from the last one
-// down, S = 2^chunk_log S + its total.
-constexpr uint32_t kFoldGroups = 4;
-template <class F>
-__global__ void __launch_bounds__(kFoldGroups * LaneGroup<F, 2>::kLanes)
-    msm_window_fold(const uint32_t* __restrict__ bits, uint32_t bit_count, const uint32_t* __restrict__ totals,
-                    uint32_t totals_stride, uint32_t levels, uint32_t chunk_log, uint32_t* __restrict__ window_sums) {
-  constexpr int XW = PointWords<F>::xyzz;
-  __shared__ __align__(16) uint32_t share[kFoldGroups][XW];
-  __shared__ __align__(16) uint32_t none[XW];  // the point at infinity
-  const uint32_t w = blockIdx.x, group = threadIdx.x / LaneGroup<F, 2>::kLanes;
-  const LaneRole<2> role{lane_role<F, 2>()};
-  const uint32_t* const z = bits + (size_t)w * (bit_count + 1) * XW;
-  const uint32_t per = (bit_count + kFoldGroups - 1) / kFoldGroups, first = group * per;
-  for (uint32_t i = threadIdx.x; i < XW; i += blockDim.x) none[i] = 0;
-  __syncthreads();
-  auto bit = [&](uint32_t k) { return k < bit_count ? z + (size_t)k * XW : none; };
-  uint32_t* const mine = share[group];
-  LanePoint<F> acc = lane_load<F>(bit(first + per - 1));
-  for (uint32_t k = per - 1; k-- > 0;) {
-    acc = lane_double(acc, role);
-    lane_store<2>(mine, acc);
-    __syncwarp();
-    lane_add<F, 2>(mine, bit(first + k), mine, true);
-    __syncwarp();
-    acc = lane_load<F>(mine);
-    __syncwarp();
-  }
-  if (per == 1) lane_store<2>(mine, acc);
-  __syncthreads();
-  if (threadIdx.x >= 32) return;
-  const bool lead = group == 0;
-  uint32_t* const sum = share[kFoldGroups - 1];  // starts as the top share
-  auto fold = [&](uint32_t doublings, const uint32_t* add) {  // sum <- 2^doublings sum + add
-    LaneChain<F> v = lane_chain<F>(sum, role);
-    for (uint32_t d = 0; d < doublings; d++) v = lane_double(v, role);
-    __syncwarp();
-    lane_store<2>(none, v, lead);  // beside what it reads; no later step needs the point at infinity
-    __syncwarp();
-    lane_add<F, 2>(none, add, sum, lead);
-    __syncwarp();
-  };
-  for (uint32_t g = kFoldGroups - 1; g-- > 0;) fold(per, share[g]);
-  lane_add<F, 2>(sum, z + (size_t)bit_count * XW, sum, lead);
-  __syncwarp();
-  for (uint32_t l = levels; l-- > 0;) fold(chunk_log, totals + ((size_t)w * totals_stride + l) * XW);
-  for (uint32_t i = threadIdx.x; i < XW; i += 32) window_sums[(size_t)w * XW + i] = sum[i];
-}
-
-// result = sum_w 2^(pos_w) S_w (msm_combine.wgsl:13-22), one group of lanes (curve_lanes.cuh) a warp; a warp's
-// other groups repeat its work. Window w is `base` bits wide, or base + 1 for w < extra (pos_w is the
-// sum of the widths below w): base = c, extra = 0 for the plain windows, the glv_window_width split for
-// GLV. Neighbours meet pairwise, 2, 4, 8 .. windows at a time counted from the top one: the top
-// windows' doublings are the chain that any order has, but only log2 W additions lie on it. Bound by
-// the latency of the doublings' products; one chain (Horner) took W - 1 additions, 5.7 us each with
-// their start of a chain (G2 8.9): G1 of 12 windows 0.169 ms, now 0.155, G2 of 24 0.495, now 0.440.
-constexpr uint32_t kCombineWindows = 32;  // 255 bits in windows of 9, at most
-template <class F>
-__global__ void __launch_bounds__(kCombineWindows / 2 * 32)
-    msm_combine_lanes(const uint32_t* __restrict__ window_sums, uint32_t windows, uint32_t base, uint32_t extra,
-                      uint32_t* __restrict__ result) {
-  constexpr int XW = PointWords<F>::xyzz;
-  __shared__ __align__(16) uint32_t part[kCombineWindows][XW];  // from the top window down
+// part[0] <- sum_i 2^pos(i) part[i] over i < count, pos falling with i, by the whole block with one
+// group of lanes (curve_lanes.cuh) a warp, at least count / 2 warps (all take part; a warp's other groups repeat
+// its work). Neighbours meet pairwise, 2, 4, 8 .. values at a time from the top: the top value's
+// doublings are the chain that any order has, but only log2 count additions lie on it.
+template <class F, class Pos>
+__device__ __forceinline__ void pairwise_horner(uint32_t (*part)[PointWords<F>::xyzz], uint32_t count, Pos pos) {
   const bool first = (threadIdx.x & 31) < LaneGroup<F, 2>::kLanes;
   const LaneRole<2> sm{lane_role<F, 2>()};
-  auto pos = [&](uint32_t w) { return w * base + min(w, extra); };
-  for (uint32_t i = threadIdx.x; i < windows * XW; i += blockDim.x) part[windows - 1 - i / XW][i % XW] = window_sums[i];
-  for (uint32_t span = 1; span < windows; span <<= 1) {
+  for (uint32_t span = 1; span < count; span <<= 1) {
     __syncthreads();
     const uint32_t high = threadIdx.x / 32 * 2 * span, low = high + span;  // this warp's pair
-    if (low >= windows) continue;
-    const uint32_t width = pos(windows - low) - pos(windows - min(low + span, windows));  // of the low part
+    if (low >= count) continue;
+    const uint32_t width = pos(low - 1) - pos(min(low + span, count) - 1);  // of the low part
     LaneChain<F> acc = lane_chain<F>(part[high], sm);
     for (uint32_t k = 0; k < width; k++) acc = lane_double(acc, sm);
     __syncwarp();
@@ -1109,6 +1049,55 @@ __global__ void __launch_bounds__(kCombineWindows / 2 * 32)
     lane_add<F, 2>(part[high], part[low], part[high], first);
   }
   __syncthreads();
+}
+
+// S_w from the Z_k and the sum of all values; then for each chunked level, from the last one down,
+// S = 2^chunk_log S + its total. Four groups of lanes that ran Horner over a share of the bits each
+// took six additions where four are left now: window sums of 12 G1 windows 0.097 ms, now 0.089, of 24 G2 windows
+// 0.265, now 0.253.
+constexpr uint32_t kFoldValues = 14;  // kMarginalMax has 12 bits
+template <class F>
+__global__ void __launch_bounds__(kFoldValues / 2 * 32)
+    msm_window_fold(const uint32_t* __restrict__ bits, uint32_t bit_count, const uint32_t* __restrict__ totals,
+                    uint32_t totals_stride, uint32_t levels, uint32_t chunk_log, uint32_t* __restrict__ window_sums) {
+  constexpr int XW = PointWords<F>::xyzz;
+  __shared__ __align__(16) uint32_t part[kFoldValues][XW];  // Z_k from the top bit down, the sum of all
+  const uint32_t w = blockIdx.x;
+  const uint32_t* const z = bits + (size_t)w * (bit_count + 1) * XW;
+  for (uint32_t i = threadIdx.x; i < (bit_count + 1) * XW; i += blockDim.x) {
+    const uint32_t k = i / XW;
+    part[k == bit_count ? k : bit_count - 1 - k][i % XW] = z[i];
+  }
+  pairwise_horner<F>(part, bit_count + 1, [&](uint32_t i) { return i == bit_count ? 0 : bit_count - 1 - i; });
+  if (threadIdx.x >= 32) return;
+  const bool first = threadIdx.x < LaneGroup<F, 2>::kLanes;
+  const LaneRole<2> role{lane_role<F, 2>()};
+  for (uint32_t l = levels; l-- > 0;) {
+    LaneChain<F> v = lane_chain<F>(part[0], role);
+    for (uint32_t d = 0; d < chunk_log; d++) v = lane_double(v, role);
+    __syncwarp();
+    lane_store<2>(part[0], v, first);
+    __syncwarp();
+    lane_add<F, 2>(part[0], totals + ((size_t)w * totals_stride + l) * XW, part[0], first);
+    __syncwarp();
+  }
+  for (uint32_t i = threadIdx.x; i < XW; i += 32) window_sums[(size_t)w * XW + i] = part[0][i];
+}
+
+// result = sum_w 2^(pos_w) S_w (msm_combine.wgsl:13-22), a warp for each pair of windows. Window w is `base`
+// bits wide, or base + 1 for w < extra (pos_w is the sum of the widths below w): base = c, extra = 0
+// for the plain windows, the glv_window_width split for GLV. Bound by the latency of the doublings'
+// products; one chain (Horner) took W - 1 additions, 5.7 us each with their start of a chain (G2
+// 8.9): G1 of 12 windows 0.169 ms, now 0.155, G2 of 24 0.495, now 0.440.
+constexpr uint32_t kCombineWindows = 32;  // 255 bits in windows of 9, at most
+template <class F>
+__global__ void __launch_bounds__(kCombineWindows / 2 * 32)
+    msm_combine_lanes(const uint32_t* __restrict__ window_sums, uint32_t windows, uint32_t base, uint32_t extra,
+                      uint32_t* __restrict__ result) {
+  constexpr int XW = PointWords<F>::xyzz;
+  __shared__ __align__(16) uint32_t part[kCombineWindows][XW];  // from the top window down
+  for (uint32_t i = threadIdx.x; i < windows * XW; i += blockDim.x) part[windows - 1 - i / XW][i % XW] = window_sums[i];
+  pairwise_horner<F>(part, windows, [&](uint32_t i) { return (windows - 1 - i) * base + min(windows - 1 - i, extra); });
   for (uint32_t i = threadIdx.x; i < XW; i += blockDim.x) result[i] = part[0][i];
 }
 
