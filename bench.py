@@ -37,19 +37,19 @@ import numpy as np  # noqa: E402
 
 METRIC = "MSM 2^20/2^24 & NTT 2^24 ms, bit-exact; batched vs plain req/s, p50/p99 ms"
 IMAD_PER_MULMOD = 264  # 8 rows x (16 product + 16 reduction multiply-adds + 1 m), field.cuh
-FP64_PER_MULMOD = 170  # double-precision instructions per Fq product in limb form, field_f64.cuh
 MULMODS_PER_MADD = 10  # madd-2008-s: 8M + 2S
-# ncu DRAM traffic (read + write bytes) per launch. msm_accumulate_f64: captured on a G1 MSM of
-# 2^22 points with the default plan (GLV split: 8.14 GB read + 0.11 GB written) and scaled by the
-# entry count to 2^24 (x4); NTT forms 0, 1 and 2: the first pass captured on the 2^24 transform.
+MULMODS_PER_AFFINE = 6  # an affine addition with a shared inversion: 5M + 1S (msm_affine.cuh)
+# ncu DRAM traffic (read + write bytes), default plans. Accumulation: the launches of its affine rounds
+# and msm_accumulate on a G1 MSM of 2^22 points, scaled by the entry count to 2^24 (x4); NTT: per
+# launch, forms 0, 1 and 2 the first pass on the 2^24 transform.
 NCU_TRAFFIC = {
-    "msm_accumulate_2^24": 33.0e9,
+    "msm_accumulate_2^24": 118.4e9,
     "ntt_form0_2^24": 1.96e9,
     "ntt_form1_2^24": 2.18e9,
-    "ntt_form2_2^24": 1.71e9,
+    "ntt_form2_2^24": 2.12e9,
 }
 # The pass kernel of each NTT form.
-NTT_KERNEL = {0: "ntt_pass", 1: "ntt_pass_f64", 2: "ntt_pass_f64s", 3: "ntt_pass_f64s", 4: "ntt_pass_f64r4"}
+NTT_KERNEL = {0: "ntt_pass", 1: "ntt_pass_f64", 2: "ntt_pass_words", 3: "ntt_pass_f64s", 4: "ntt_pass_f64r4"}
 
 
 def parse():
@@ -346,10 +346,12 @@ def run_ours(a, d: Dist) -> dict | None:
 
     # ---- rooflines
     acc_ms = st24.get("accumulate", float("nan"))
-    acc_ops = entries.value * MULMODS_PER_MADD * IMAD_PER_MULMOD
+    # the plan's affine rounds halve what is left for mixed additions each (MsmPlan::affine_rounds)
+    most = (1 << a.log_msm) * 2 * -(-128 // c24)
+    rounds = 4 if most >= 1 << 28 else 3 if most >= 1 << 26 else 2 if most >= 1 << 23 else 0
+    mulmods_per_entry = MULMODS_PER_AFFINE * (1 - 2.0 ** -rounds) + MULMODS_PER_MADD * 2.0 ** -rounds
+    acc_ops = entries.value * mulmods_per_entry * IMAD_PER_MULMOD
     acc_achieved = acc_ops / (acc_ms * 1e-3)
-    acc_fp64 = entries.value * MULMODS_PER_MADD * FP64_PER_MULMOD / (acc_ms * 1e-3)
-    acc_variant = msm24.params()["variant"]
     n_pass = len(stn)
     ntt_pass_ms = sum(stn.values()) / max(n_pass, 1)  # mean pass duration (forward and inverse)
     ntt_bytes = 64 * nn  # each pass reads and writes 32 B per element
@@ -391,21 +393,20 @@ def run_ours(a, d: Dist) -> dict | None:
                       f"msm_2^{a.log_msm_small}": {k: round(v, 4) for k, v in st20.items()},
                       f"ntt_2^{a.log_ntt}": {k: round(v, 4) for k, v in stn.items()}},
         "roofline": {
-            "kernel": (f"msm_accumulate_f64 (G1 MSM 2^{a.log_msm}; Fq products on the FP64 pipe)" if acc_variant >= 3
-                       else f"msm_accumulate<Fq> (G1 MSM 2^{a.log_msm})"),
+            "kernel": f"msm_affine_* ({rounds} rounds) and msm_accumulate<Fq> (G1 MSM 2^{a.log_msm})",
             "bound": "imad",
             "achieved": round(acc_achieved / 1e12, 3),
             "peak": round(imad_peak / 1e12, 3),
             "unit": "T int-mul-add/s",
             "frac": round(acc_achieved / imad_peak, 4),
             "traffic": NCU_TRAFFIC["msm_accumulate_2^24"],
-            "algorithmic": f"{entries.value} nonzero digits x {MULMODS_PER_MADD} Fq products x "
-                           f"{IMAD_PER_MULMOD} 32-bit multiply-adds (the integer-product equivalent of the work)",
+            "algorithmic": f"{entries.value} nonzero digits x {mulmods_per_entry} Fq products ({MULMODS_PER_AFFINE} an "
+                           f"affine, {MULMODS_PER_MADD} a mixed addition) x {IMAD_PER_MULMOD} 32-bit multiply-adds",
             "peak_source": "measured in this run: best of mad.lo / mad.hi / carry-chain probes "
                            "(zkg_bench_integer_pipe)",
-            "fp64_pipe": {"achieved": round(acc_fp64 / 1e12, 3), "peak": round(peaks["dfma"] / 1e12, 3),
-                          "unit": "T FP64 instr/s", "frac": round(acc_fp64 / peaks["dfma"], 4),
-                          "algorithmic": f"{FP64_PER_MULMOD} FP64 instructions per Fq product"},
+            "product_rate": {"achieved": round(acc_achieved / IMAD_PER_MULMOD / 1e9, 2),
+                             "peak": round(peaks["fq_mulmod"] / 1e9, 2), "unit": "G Fq products/s",
+                             "frac": round(acc_achieved / IMAD_PER_MULMOD / peaks["fq_mulmod"], 4)},
         },
         "roofline_ntt": {
             "kernel": (f"{NTT_KERNEL.get(ntt.params()['variant'], 'ntt_pass')} (Fr NTT 2^{a.log_ntt}, {n_pass} passes, "
@@ -417,17 +418,17 @@ def run_ours(a, d: Dist) -> dict | None:
             "frac": round(ntt_gbs / hbm_peak, 4),
             "peak_source": hbm_src,
             "traffic": NCU_TRAFFIC.get(f"ntt_form{ntt.params()['variant']}_2^24"),
-            "algorithmic": "64 B per element per pass (read + write); the first pass also reads its staged "
-                           "twiddles, 40 B per element (form 2)",
+            "algorithmic": "64 B per element per pass (read + write), beside the passes' twiddle tables",
             "transform_frac_of_hbm": round((ntt_bytes * n_pass / (sum(stn.values()) * 1e-3) / 1e9) / hbm_peak, 4),
             "product_rate": {
                 "achieved": round(ntt_products / (sum(stn.values()) * 1e-3) / 1e9, 2),
-                "peak": round(peaks["fq_mulmod_fp64"] / 1e9, 2),
+                "peak": round(peaks["fq_mulmod"] / 1e9, 2),
                 "unit": "G Fr products/s",
-                "frac": round(ntt_products / (sum(stn.values()) * 1e-3) / peaks["fq_mulmod_fp64"], 4),
+                "frac": round(ntt_products / (sum(stn.values()) * 1e-3) / peaks["fq_mulmod"], 4),
                 "algorithmic": f"{ntt_products} twiddle products per forward transform (log2(n) n/2 butterflies "
                                "less the n - 1 with twiddle 1); peak: the measured rate of independent "
-                               "double-precision-limb Montgomery products (zkg_bench_integer_pipe variant 11)",
+                               "Montgomery products (zkg_bench_integer_pipe variant 3; a product by a twiddle with "
+                               "a precomputed quotient takes 107 of its 132 multiply-add slots)",
             },
         },
         "integer_pipe_probe": {k: round(v / 1e12, 3) for k, v in peaks.items()},
