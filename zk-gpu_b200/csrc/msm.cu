@@ -64,7 +64,8 @@ uint32_t auto_seg_len(size_t entries, int group, int sms) {
 }
 
 // Entries of one batch of affine rounds. A batch's points between rounds take 48 bytes an entry (G2 96),
-// and there are two batches' scratch; G1 2^24 40.4 ms with batches of 2^24, 39.2 with 2^25.
+// and there are two batches' scratch; G1 2^24 40.4 ms with batches of 2^24, 39.2 with 2^25. Each stream has as
+// many batches: accumulation at G1 2^22 8.77 ms in three of them, 8.45 in two.
 static size_t affine_batch(int group) { return (size_t)1 << (group == ZKG_G1 ? 25 : 24); }
 
 // Pairs per thread of a round over `pairs` pairs: about 32, such that the threads fill whole waves of
@@ -184,7 +185,9 @@ void MsmPlan::layout_rounds(uint32_t group_log) {
   tile_sums.alloc(scan_tiles_n, "msm scan tiles");
   sorted.alloc(rounds.groups << group_log, "msm sorted");
   if (group_log) {
-    batch_groups = (uint32_t)std::min<size_t>((rounds.groups + 1) / 2, affine_batch(group) >> group_log);  // one for each stream
+    // as many batches for each stream, of affine_batch's size and an eighth more at most
+    const size_t two = (affine_batch(group) >> group_log) * 9 / 4, twos = (rounds.groups + two - 1) / two;
+    batch_groups = (uint32_t)((rounds.groups + 2 * twos - 1) / (2 * twos));
     affine_sums.alloc(rounds.groups * affine_words(), "msm affine sums");
     size_t threads = 0;  // of the largest round
     for (uint32_t r = 1; r <= group_log; r++) {

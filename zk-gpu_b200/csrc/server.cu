@@ -128,7 +128,7 @@ size_t Server::estimate_bytes(uint32_t log_m, bool rounds) const {
     // affine rounds: a point per four entries, and two batches' points between rounds
     const size_t affine = !rounds || entries < (1u << 22)
                               ? 0
-                              : xw / 2 * (entries / 4 + 2 * S + std::min(entries / 2, (size_t)1 << 25) * 3 / 2);
+                              : xw / 2 * (entries / 4 + 2 * S + std::min(entries / 2, (size_t)1 << 25) * 7 / 4);
     // counts, slot starts, cursors; sorted entries, ranks and digits; buckets; heads; running
     // sums; the GLV bases (phi of the m points)
     return 4 * (3 * S + entries * 5 / 2 + S * xw + (heads + heads / 16 + 2) * (xw + 1) + 8 * W * B / 16 * xw / 8 +
