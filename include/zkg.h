@@ -11,7 +11,8 @@
  *    panics (tests/invalid_inputs.rs:9-50), so a binding can panic with it unchanged.
  *  - Memory format (unchanged from the reference): 8 little-endian u32 words per field
  *    element; affine points are x then y, Fq2 coordinates a then b (x = a + b*u, u^2 = -1);
- *    the point at infinity is all-zero words (src/msm.rs:182-183, src/group.rs:59-69).
+ *    the point at infinity is all-zero words (src/msm.rs:182-183, src/group.rs:59-69). Coordinates
+ *    are below q and transform data below r; with other words a call's result means nothing.
  *  - Work is queued on the context's single ordered stream and runs asynchronously until a
  *    read or zkg_ctx_sync, like the reference's wgpu queue (src/gpu.rs:151-155).
  *  - Results of the MSM are XYZZ points in Montgomery form with R = 2^256 (the reference's

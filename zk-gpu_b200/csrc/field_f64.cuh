@@ -333,12 +333,14 @@ __device__ __forceinline__ FqD fqd_sub2(const FqD& a, const FqD& b, const FqD& c
 }
 
 // x (below 16m) -> x - q m in [0, 2m), q from the top limb (q never exceeds floor(x / m), and
-// falls short of it by at most one). kp holds k m, k = 0..15, in normalized limbs.
+// falls short of it by at most one). kp holds k m, k = 0..15, in normalized limbs. Words that a
+// caller left at or above the modulus can bring x out of that range (a negative x gives a q that
+// wraps): the sum is meaningless then, but the row read stays in the table.
 template <class L = FqLimbs>
 __device__ __forceinline__ FqD fqd_reduce(const FqD& x, const MultiplesOf<L>* __restrict__ kp) {
   const double qm = __fma_rd(x.l[4], kInvP4, kFloorMagic);
-  const int q = (int)((uint64_t)__double_as_longlong(qm) - (uint64_t)__double_as_longlong(kFloorMagic));
-  const double* m = kp->v[q];
+  const uint32_t q = (uint32_t)((uint64_t)__double_as_longlong(qm) - (uint64_t)__double_as_longlong(kFloorMagic));
+  const double* m = kp->v[min(q, 15u)];
   double t[5];
 #pragma unroll
   for (int j = 0; j < 5; j++) t[j] = __dsub_rn(x.l[j], __ldg(m + j));
