@@ -684,9 +684,10 @@ int zkg_msm_last_entries(zkg_msm* msm, uint64_t* entries) {
     need(entries, "entries");
     use(msm->plan.ctx);
     uint32_t v = 0;
-    check_cuda(cudaMemcpyAsync(&v, msm->plan.counts.ptr + msm->plan.active_slots(), 4, cudaMemcpyDeviceToHost,
-                               msm->plan.ctx->stream),
-               "entry count");
+    if (msm->plan.entries_at != MsmPlan::kNoEntries)
+      check_cuda(cudaMemcpyAsync(&v, msm->plan.counts.ptr + msm->plan.entries_at, 4, cudaMemcpyDeviceToHost,
+                                 msm->plan.ctx->stream),
+                 "entry count");
     check_cuda(cudaStreamSynchronize(msm->plan.ctx->stream), "entry count");
     *entries = v;
   });

@@ -149,6 +149,7 @@ void MsmPlan::layout() {
   windows = glv ? (128 + c - 1) / c : (255 + c - 1) / c;
   half = 1u << (c - 1);
   slots = (size_t)windows * half;
+  entries_at = kNoEntries;
   if (const uint32_t group_log = affine_rounds(windows * np)) {
     try {
       layout_rounds(group_log);
@@ -590,6 +591,7 @@ const char* MsmPlan::stage_name(int which) {
 // slice of the bases (a fixed-base plan has one pass) and scalars.
 void MsmPlan::begin_pass(size_t off, const uint32_t*& bases, const uint32_t*& scalars) {
   run_n = std::min(chunk, n - off);
+  entries_at = active_slots();
   first_pass = off == 0;
   combine_out = first_pass ? result.ptr : partial.ptr;
   bases += off * affine_words();

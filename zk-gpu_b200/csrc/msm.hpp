@@ -74,6 +74,10 @@ struct MsmPlan {
   // results are added (the reference's limit, n < 2^31, is kept). The plan's scratch is sized
   // for one pass, so a smaller chunk (zkg_msm_set_chunk) also bounds its device memory.
   size_t chunk = 0, run_n = 0;  // run_n: the points of the pass being queued
+  // Where the last pass left its entry count in `counts` (the switches between runs move active_slots());
+  // kNoEntries before a run and after a change of layout.
+  static constexpr size_t kNoEntries = ~(size_t)0;
+  size_t entries_at = kNoEntries;
   size_t chunk_req = 0;         // 0: the largest pass the mode allows
   size_t max_chunk() const;
   void set_chunk(size_t points);
