@@ -174,6 +174,18 @@ int zkg_msm_windows(const zkg_msm *msm, uint32_t *windows, int *glv);
  * the same point for every slice size. */
 int zkg_msm_set_chunk(zkg_msm *msm, size_t points);
 int zkg_msm_passes(const zkg_msm *msm, size_t *chunk, size_t *passes);
+/* Affine rounds (no reference counterpart): from 2^23 (window, point) entries on (G2 2^22), a plan in its
+ * default form adds the entries of a bucket pairwise, as affine points with shared inversions, in two to
+ * four rounds before the bucket sums. Their scratch is one to four times the rest of the plan's memory
+ * (G1 2^20 320 MiB without it, 1220 with; 2^24 3.8 and 7.9 GiB). It is taken where the device has room and
+ * given back for the plan's lifetime when a later allocation of this library on the device fails, unless
+ * a graph captured with the plan may hold it; results do not change, runs are then slower by the
+ * rounds' gain. zkg_msm_set_rounds(msm, 0) makes the plan do without it, for memory that other
+ * allocators want; 1 lays it out again where it fits (re-sizes the scratch, synchronising with queued work; batches
+ * that hold the plan have to be made anew). zkg_msm_rounds reports the rounds of a run and the bytes of
+ * their scratch. */
+int zkg_msm_set_rounds(zkg_msm *msm, int enable);
+int zkg_msm_rounds(const zkg_msm *msm, uint32_t *rounds, size_t *bytes);
 int zkg_msm_params(const zkg_msm *msm, uint32_t *c, uint32_t *item_points, int *variant);
 /* Msm::run (src/msm.rs:284-298): queue sum(scalars[i] * bases[i]); scalars are 8 plain u32
  * words each. *result is a borrowed handle to the plan's XYZZ result (32 words G1, 64 words G2,

@@ -443,6 +443,22 @@ int zkg_msm_set_chunk(zkg_msm* msm, size_t points) {
   });
 }
 
+int zkg_msm_set_rounds(zkg_msm* msm, int enable) {
+  return guard([&] {
+    need(msm, "msm");
+    msm->plan.set_rounds(enable != 0);
+  });
+}
+
+int zkg_msm_rounds(const zkg_msm* msm, uint32_t* rounds, size_t* bytes) {
+  return guard([&] {
+    need(msm, "msm");
+    std::lock_guard<std::mutex> lock(msm->plan.queue_mu);
+    if (rounds) *rounds = msm->plan.run_rounds();
+    if (bytes) *bytes = msm->plan.rounds_bytes();
+  });
+}
+
 int zkg_msm_passes(const zkg_msm* msm, size_t* chunk, size_t* passes) {
   return guard([&] {
     need(msm, "msm");
@@ -471,6 +487,7 @@ int zkg_test_glv_split(zkg_ctx* ctx, const uint32_t* scalars, size_t count, uint
 int zkg_msm_params(const zkg_msm* msm, uint32_t* c, uint32_t* item_points, int* variant) {
   return guard([&] {
     need(msm, "msm");
+    std::lock_guard<std::mutex> lock(msm->plan.queue_mu);
     if (c) *c = msm->plan.c;
     if (item_points) *item_points = msm->plan.segments().seg_len;
     if (variant) *variant = msm->plan.acc_variant;

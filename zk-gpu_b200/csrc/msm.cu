@@ -143,8 +143,87 @@ void MsmPlan::set_chunk(size_t points) {
   }
 }
 
+// The plans that hold spare memory, of every device.
+struct SpareList {
+  std::mutex mu;
+  std::vector<MsmPlan*> plans;
+};
+static SpareList& spare_list() {
+  static SpareList* list = new SpareList;  // outlives plans of any lifetime
+  return *list;
+}
+void SpareEntry::list(MsmPlan* p) {
+  SpareList& l = spare_list();
+  std::lock_guard<std::mutex> lock(l.mu);
+  plan = p;
+  l.plans.push_back(p);
+}
+void SpareEntry::unlist() {
+  if (!plan) return;
+  SpareList& l = spare_list();
+  std::lock_guard<std::mutex> lock(l.mu);
+  l.plans.erase(std::remove(l.plans.begin(), l.plans.end(), plan), l.plans.end());
+  plan = nullptr;
+}
+
+bool give_back_spare(size_t bytes) {
+  int device = 0;
+  size_t free_bytes = 0, total = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) return false;
+  SpareList& l = spare_list();
+  std::lock_guard<std::mutex> lock(l.mu);
+  size_t all = free_bytes;
+  for (const MsmPlan* p : l.plans)
+    if (p->ctx->device == device) all += p->spare_bytes();
+  if (all < bytes) return false;
+  for (MsmPlan* p : l.plans)
+    if (p->ctx->device == device && p->give_back()) return true;
+  return false;
+}
+
+void MsmPlan::release_rounds() {
+  affine_sums.release();
+  for (AffineLane& lane : affine_lane) {
+    lane.inverses.release();
+    lane.mid[0].release();
+    lane.mid[1].release();
+  }
+}
+
+size_t MsmPlan::rounds_bytes() const {
+  size_t words = affine_sums.words;
+  for (const AffineLane& lane : affine_lane) words += lane.inverses.words + lane.mid[0].words + lane.mid[1].words;
+  return 4 * words;
+}
+
+void MsmPlan::drop_rounds() {
+  rounds = plain;
+  release_rounds();  // cudaFree waits for the runs that use it
+}
+
+size_t MsmPlan::spare_bytes() const {
+  std::lock_guard<std::mutex> lock(queue_mu);
+  return captured ? 0 : rounds_bytes();
+}
+
+size_t MsmPlan::give_back() {
+  std::lock_guard<std::mutex> lock(queue_mu);
+  const size_t bytes = captured ? 0 : rounds_bytes();
+  if (bytes) drop_rounds();
+  return bytes;
+}
+
+void MsmPlan::set_rounds(bool enable) {
+  use(ctx);
+  affine = enable;
+  layout();
+}
+
 // Where the affine rounds' scratch does not fit the device beside the rest, the plan goes without.
 void MsmPlan::layout() {
+  spare.unlist();
+  captured = false;
+  release_rounds();
   const size_t np = glv ? 2 * chunk : chunk;
   windows = glv ? (128 + c - 1) / c : (255 + c - 1) / c;
   half = 1u << (c - 1);
@@ -153,10 +232,11 @@ void MsmPlan::layout() {
   if (const uint32_t group_log = affine_rounds(windows * np)) {
     try {
       layout_rounds(group_log);
+      spare.list(this);
       return;
     } catch (const Error& e) {
       if (e.code != ZKG_ENOMEM) throw;
-      cudaGetLastError();
+      release_rounds();
     }
   }
   layout_rounds(0);
@@ -185,36 +265,6 @@ void MsmPlan::layout_rounds(uint32_t group_log) {
   if (scan_tiles_n > (uint32_t)kScanTile) fail(ZKG_EINVAL, "too many bucket slots");
   tile_sums.alloc(scan_tiles_n, "msm scan tiles");
   sorted.alloc(rounds.groups << group_log, "msm sorted");
-  if (group_log) {
-    // as many batches for each stream, of affine_batch's size and an eighth more at most
-    const size_t two = (affine_batch(group) >> group_log) * 9 / 4, twos = (rounds.groups + two - 1) / two;
-    batch_groups = (uint32_t)((rounds.groups + 2 * twos - 1) / (2 * twos));
-    affine_sums.alloc(rounds.groups * affine_words(), "msm affine sums");
-    size_t threads = 0;  // of the largest round
-    for (uint32_t r = 1; r <= group_log; r++) {
-      const size_t pairs = (size_t)batch_groups << (group_log - r);
-      const size_t per = affine_per_thread(pairs, group, ctx->sm_count);
-      threads = std::max<size_t>(threads, (size_t)grid_for((pairs + per - 1) / per, kAffineThreads) * kAffineThreads);
-    }
-    for (AffineLane& lane : affine_lane) {
-      lane.inverses.alloc(threads * (affine_words() / 2), "msm affine inverses");
-      for (uint32_t k = 0; k < 2; k++) {  // rounds 1 and 2 write the largest arrays
-        if (group_log > k + 1)
-          lane.mid[k].alloc(((size_t)batch_groups << (group_log - 1 - k)) * affine_words(), "msm affine points");
-        else lane.mid[k].release();
-      }
-    }
-    if (!side.stream) check_cuda(cudaStreamCreateWithFlags(&side.stream, cudaStreamNonBlocking), "msm side stream");
-    if (!side.fork) check_cuda(cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming), "msm side event");
-    if (!side.join) check_cuda(cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming), "msm side event");
-  } else {
-    affine_sums.release();
-    for (AffineLane& lane : affine_lane) {
-      lane.inverses.release();
-      lane.mid[0].release();
-      lane.mid[1].release();
-    }
-  }
   if (c <= 16) {
     ranks.alloc(max_entries, "msm ranks");
     digits.alloc((max_entries + 1) / 2, "msm ranked digits");  // 16 bits per entry
@@ -266,6 +316,28 @@ void MsmPlan::layout_rounds(uint32_t group_log) {
   else glv_bases.release();
   if (passes() > 1) partial.alloc(xw, "msm pass result");
   else partial.release();
+  if (group_log) {  // last, when the rest has what it needs
+    // as many batches for each stream, of affine_batch's size and an eighth more at most
+    const size_t two = (affine_batch(group) >> group_log) * 9 / 4, twos = (rounds.groups + two - 1) / two;
+    batch_groups = (uint32_t)((rounds.groups + 2 * twos - 1) / (2 * twos));
+    affine_sums.alloc(rounds.groups * affine_words(), "msm affine sums", true);
+    size_t threads = 0;  // of the largest round
+    for (uint32_t r = 1; r <= group_log; r++) {
+      const size_t pairs = (size_t)batch_groups << (group_log - r);
+      const size_t per = affine_per_thread(pairs, group, ctx->sm_count);
+      threads = std::max<size_t>(threads, (size_t)grid_for((pairs + per - 1) / per, kAffineThreads) * kAffineThreads);
+    }
+    for (AffineLane& lane : affine_lane) {
+      lane.inverses.alloc(threads * (affine_words() / 2), "msm affine inverses", true);
+      for (uint32_t k = 0; k < 2; k++) {  // rounds 1 and 2 write the largest arrays
+        if (group_log > k + 1)
+          lane.mid[k].alloc(((size_t)batch_groups << (group_log - 1 - k)) * affine_words(), "msm affine points", true);
+      }
+    }
+    if (!side.stream) check_cuda(cudaStreamCreateWithFlags(&side.stream, cudaStreamNonBlocking), "msm side stream");
+    if (!side.fork) check_cuda(cudaEventCreateWithFlags(&side.fork, cudaEventDisableTiming), "msm side event");
+    if (!side.join) check_cuda(cudaEventCreateWithFlags(&side.join, cudaEventDisableTiming), "msm side event");
+  }
 }
 
 size_t MsmPlan::xyzz_words() const { return group == ZKG_G1 ? 32 : 64; }
@@ -599,6 +671,12 @@ void MsmPlan::begin_pass(size_t off, const uint32_t*& bases, const uint32_t*& sc
 }
 
 void MsmPlan::enqueue(const uint32_t* bases, const uint32_t* scalars, cudaStream_t s) {
+  std::lock_guard<std::mutex> lock(queue_mu);
+  if (segments().group_log && !captured) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    check_cuda(cudaStreamIsCapturing(s, &status), "stream capture status");
+    captured = status != cudaStreamCaptureStatusNone;
+  }
   for (size_t off = 0; off < n; off += chunk) {
     const uint32_t *b = bases, *sc = scalars;
     begin_pass(off, b, sc);
@@ -621,6 +699,7 @@ void MsmPlan::run(const zkg_buf* bases, const zkg_buf* scalars) {
 std::vector<std::pair<std::string, double>> MsmPlan::profile(const zkg_buf* bases, const zkg_buf* scalars) {
   check_buffers(bases, scalars);
   use(ctx);
+  std::lock_guard<std::mutex> lock(queue_mu);
   std::vector<std::pair<std::string, double>> out;
   cudaEvent_t a, b;
   check_cuda(cudaEventCreate(&a), "event");

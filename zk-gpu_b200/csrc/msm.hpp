@@ -1,5 +1,6 @@
 // MSM plan (host side of Msm, src/msm.rs:25-298).
 #pragma once
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -19,6 +20,16 @@ void fixed_base_table(zkg_ctx* ctx, int group, const zkg_buf* bases, size_t n, u
 // words each) and their signs (1 word each), to host memory.
 void glv_split(zkg_ctx* ctx, const uint32_t* scalars, size_t count, uint32_t* out);
 
+struct MsmPlan;
+
+// A plan's place among those that hold spare memory (give_back_spare); leaves it when destroyed.
+struct SpareEntry {
+  MsmPlan* plan = nullptr;
+  void list(MsmPlan* p);
+  void unlist();
+  ~SpareEntry() { unlist(); }
+};
+
 struct MsmPlan {
   enum Stage {
     kStageCount,
@@ -36,7 +47,7 @@ struct MsmPlan {
   int group;
   size_t n;
   uint32_t c, windows = 0, half = 0;
-  bool affine;  // may have affine rounds (their scratch doubles the plan's or more)
+  bool affine;  // may have affine rounds (their scratch doubles the plan's memory or more)
   // Accumulation kernel form: 0 = integer field products inlined, 1 = through one out-of-line
   // product, 2 = out of line, independent products two per call (G2: one reduction per component of
   // an Fq2 product), 3 / 5 / 6 = bucket arithmetic in
@@ -90,6 +101,8 @@ struct MsmPlan {
   // (msm_affine.cuh) have made one point, or the entries themselves (group_log = 0); in segments of
   // seg_len, one partial sum (head) each at most, merged in merge_levels launches. The rounds belong to the plan's own
   // accumulation form; the scratch holds both layouts, so that switching the form moves nothing.
+  // The rounds' own scratch (affine_sums, affine_lane) is spare memory: taken where the device has
+  // room, given back when an allocation fails for want of it (G1 2^20 320 MiB without it, 1220 with).
   struct Segments {
     uint32_t group_log = 0, seg_len = 0, merge_levels = 0;
     size_t groups = 0, heads = 0;
@@ -141,6 +154,15 @@ struct MsmPlan {
   void check_buffers(const zkg_buf* bases, const zkg_buf* scalars) const;
   void set_fixed_base(bool enable);
   void set_glv(bool enable);
+  // Whether the plan may have affine rounds; lays the scratch out anew.
+  void set_rounds(bool enable);
+  uint32_t run_rounds() const { return segments().group_log; }  // of a run as the plan is now
+  // Frees the rounds' scratch and goes on without them (queued runs finish first); the rest of the
+  // scratch stays where it is. Called under queue_mu by others than the plan's user.
+  void drop_rounds();
+  size_t rounds_bytes() const;    // of the rounds' scratch
+  size_t spare_bytes() const;     // the same, or 0 while a captured graph may hold it
+  size_t give_back();             // drop_rounds if there are spare bytes; their number
   // Queues every stage on stream s (no host synchronisation).
   void enqueue(const uint32_t* bases, const uint32_t* scalars, cudaStream_t s);
   void run(const zkg_buf* bases, const zkg_buf* scalars);
@@ -164,6 +186,15 @@ struct MsmPlan {
   template <int AGG>
   void rank(const uint32_t* bases, const uint32_t* scalars, cudaStream_t s);
   uint32_t item_points_req = 0;
+  void release_rounds();
+
+ public:
+  // Held while a run is queued and while the rounds' scratch is given back, by whichever thread.
+  mutable std::mutex queue_mu;
+
+ private:
+  bool captured = false;  // a graph may hold the rounds' scratch
+  SpareEntry spare;       // last: the plan is off the list before its arrays go
 };
 
 }  // namespace zkg

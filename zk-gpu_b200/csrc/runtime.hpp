@@ -97,10 +97,23 @@ inline void wait_reads(const zkg_buf* b, cudaStream_t stream) {
   if (b && b->pending_read) check_cuda(cudaStreamWaitEvent(stream, b->pending_read, 0), "cudaStreamWaitEvent");
 }
 
-inline uint32_t* device_alloc(size_t bytes, const char* what) {
+// Gives back, on the current device, memory that one plan holds for speed alone (MsmPlan::give_back);
+// false, and nothing is given back, when all such memory and what is free cannot make up `bytes`.
+bool give_back_spare(size_t bytes);
+
+// A failed allocation is tried again without the plans' spare memory, so that what fits beside the
+// memory they need is not refused for the sake of what they can do without. `spare`: the allocation is
+// itself of that kind, and takes it from nobody.
+inline uint32_t* device_alloc(size_t bytes, const char* what, bool spare = false) {
   void* p = nullptr;
   if (bytes == 0) bytes = 16;
-  check_cuda(cudaMalloc(&p, bytes), what);
+  cudaError_t e = cudaMalloc(&p, bytes);
+  while (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    if (spare || !give_back_spare(bytes)) break;
+    e = cudaMalloc(&p, bytes);
+  }
+  check_cuda(e, what);
   return static_cast<uint32_t*>(p);
 }
 
@@ -112,9 +125,9 @@ struct DeviceArray {
   DeviceArray(const DeviceArray&) = delete;
   DeviceArray& operator=(const DeviceArray&) = delete;
   ~DeviceArray() { release(); }
-  void alloc(size_t w, const char* what) {
+  void alloc(size_t w, const char* what, bool spare = false) {
     release();
-    ptr = device_alloc(w * 4, what);
+    ptr = device_alloc(w * 4, what, spare);
     words = w;
   }
   void release() {

@@ -86,6 +86,8 @@ SIGNATURES = {
                                        ctypes.POINTER(ctypes.c_int)]),
     "zkg_zkey_upload": (ctypes.c_int, [vp, vp, ctypes.c_uint32, ctypes.POINTER(vp)]),
     "zkg_ntt_forward_quotient": (ctypes.c_int, [vp, vp, vp, vp, u32p]),
+    "zkg_msm_set_rounds": (ctypes.c_int, [vp, ctypes.c_int]),
+    "zkg_msm_rounds": (ctypes.c_int, [vp, ctypes.POINTER(ctypes.c_uint32), ctypes.POINTER(ctypes.c_size_t)]),
     "zkg_msm_params": (ctypes.c_int, [vp, ctypes.POINTER(ctypes.c_uint32), ctypes.POINTER(ctypes.c_uint32),
                                       ctypes.POINTER(ctypes.c_int)]),
     "zkg_msm_run": (ctypes.c_int, [vp, vp, vp, ctypes.POINTER(vp)]),

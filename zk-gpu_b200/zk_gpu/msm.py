@@ -94,6 +94,17 @@ class Msm:
         check(lib().zkg_msm_passes(self._h, ctypes.byref(ch), ctypes.byref(ps)))
         return ch.value, ps.value
 
+    def set_rounds(self, enable: bool = True) -> None:
+        """Affine rounds before the bucket sums (large plans, on by default where the device has room);
+        off, the plan holds a half to a fifth of the memory. The result does not change."""
+        check(lib().zkg_msm_set_rounds(self._h, int(enable)))
+
+    def rounds(self) -> tuple[int, int]:
+        """(affine rounds of a run, bytes of their scratch)."""
+        r, b = ctypes.c_uint32(), ctypes.c_size_t()
+        check(lib().zkg_msm_rounds(self._h, ctypes.byref(r), ctypes.byref(b)))
+        return r.value, b.value
+
     def set_glv(self, enable: bool = True) -> None:
         """G1: split every scalar as k1 + k2 lambda (mod r) and run over P_i and phi(P_i) with
         ceil(128 / c) windows; the same result as the plain MSM."""
