@@ -293,7 +293,9 @@ int zkg_zkey_upload(zkg_ctx *ctx, const zkg_zkey *zkey, uint32_t section, zkg_bu
  * zkg_ntt_set_variant picks a plan's butterfly form: 0 = 32-bit integer products, radix 2 (tiles of
  * 2^11 elements), 1 = double-precision limbs, products on the FP64 pipe (tiles of 2^10), 2 = integer
  * words, radix 4 in registers (default), 3 and 4 = double-precision limbs with staged twiddles, radix
- * 2 and 4; it resets the pass split to the form's default (at most 9 stages per pass in form 0, 8 in
+ * 2 and 4. Form 2's tables take 64 bytes per twiddle and direction, those of forms 3 and 4 take 40 (2^24:
+ * 2.5 and 1.8 GiB of plan memory): a plan whose form 2 does not fit the device is made in form 3.
+ * zkg_ntt_set_variant resets the pass split to the form's default (at most 9 stages per pass in form 0, 8 in
  * the others). zkg_ntt_set_max_stages picks the pass split (at most max_stages, 6..=11 for form 0,
  * 6..=10 for the others, stages per shared-memory pass); zkg_ntt_params reports form, split and passes.
  * zkg_tune_ntt times every form and each split on `data` (forward + inverse, which leaves the

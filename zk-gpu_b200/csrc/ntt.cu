@@ -593,8 +593,14 @@ NttPlan::NttPlan(zkg_ctx* c, uint32_t log_n_) : ctx(c), log_n(log_n_) {
   set_pass_smem_limits();
   // Integer words by default at every size. Measured on B200, us per forward transform, beside two
   // double-precision butterflies per thread step (form 3): 2^12 19.5 / 39, 2^16 24.7 / 47, 2^20
-  // 175 / 300, 2^24 2853 / 5283.
-  set_variant(2);
+  // 175 / 300, 2^24 2853 / 5283. Where its tables (64 bytes per twiddle and direction) do not fit the
+  // device, form 3's may (40 bytes).
+  try {
+    set_variant(2);
+  } catch (const Error& e) {
+    if (e.code != ZKG_ENOMEM) throw;
+    set_variant(3);
+  }
 }
 
 uint32_t NttPlan::tile_log() const { return variant != 0 ? kTileLogD : kTileLog; }
@@ -620,14 +626,31 @@ bool NttPlan::set_variant(int v) {
     check_launch("ntt_twiddles_to_limbs");
     check_cuda(cudaStreamSynchronize(ctx->setup), "ntt twiddle limbs");
   }
-  variant = v;
   // Pass split: one tile when it fits, else passes of near-equal size, at most 9 stages each
-  // (integer form, tiles of 2^11) or 8 (double-precision forms, tiles of 2^10).
-  set_max_stages(v != 0 ? kMaxStagesPerPassD : kMaxStagesPerPass);
+  // (form 0, tiles of 2^11) or 8 (the others, tiles of at most 2^10).
+  choose(v, v != 0 ? kMaxStagesPerPassD : kMaxStagesPerPass);
   return true;
 }
 
-bool NttPlan::set_max_stages(uint32_t ms) {
+bool NttPlan::set_max_stages(uint32_t ms) { return choose(variant, ms); }
+
+// Form v in passes of at most ms stages; where its tables do not fit the device, the form and split
+// of before are laid out again (in the memory that they had) and the error goes on.
+bool NttPlan::choose(int v, uint32_t ms) {
+  const int old = variant;
+  const uint32_t old_stages = max_stages;
+  const bool built = !passes.empty();
+  variant = v;
+  try {
+    return split(ms);
+  } catch (...) {
+    variant = old;
+    if (built) split(old_stages);
+    throw;
+  }
+}
+
+bool NttPlan::split(uint32_t ms) {
   const uint32_t tlog = tile_log();
   const uint32_t def = variant != 0 ? kMaxStagesPerPassD : kMaxStagesPerPass;
   if (ms < 6 || ms > tlog) return false;

@@ -64,6 +64,8 @@ struct NttPlan {
   void build_twiddles(DeviceArray (&seed)[2], DeviceArray& out);
   // Forms 3 and 4, and form 2: one table per pass and direction, for the split in `passes`.
   void build_stage_tables();
+  bool choose(int v, uint32_t ms);
+  bool split(uint32_t ms);
   void build_words_tables();
   std::vector<uint32_t> words_tile;  // log2 of the tile, per pass
   std::vector<std::unique_ptr<DeviceArray>> stage_tw[2];

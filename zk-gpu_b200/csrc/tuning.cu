@@ -80,10 +80,19 @@ std::vector<NttChoice> tune_ntt(zkg_ctx* ctx, uint32_t log_n, zkg_buf* data, int
   if (data->words < ((size_t)8 << log_n)) fail(ZKG_ESIZE, "data buffer too small for the transform");
   std::vector<NttChoice> out;
   for (int v = 0; v <= 4; v++) {
-    plan->set_variant(v);
+    // false for a form or split that the plan does not take or whose tables do not fit the device
+    auto fits = [&](auto set) {
+      try {
+        return set();
+      } catch (const Error& e) {
+        if (e.code != ZKG_ENOMEM) throw;
+        return false;
+      }
+    };
+    if (!fits([&] { return plan->set_variant(v); })) continue;
     const uint32_t tlog = plan->tile_log();
     for (uint32_t s = 6; s <= tlog; s++) {
-      if (!plan->set_max_stages(s)) continue;
+      if (!fits([&] { return plan->set_max_stages(s); })) continue;
       if (plan->passes.size() == 1 && s != tlog) continue;  // one tile: every split is the same
       double ms = time_ms(ctx->stream, reps, [&] {
         plan->enqueue(data->ptr, false, ctx->stream);
