@@ -346,7 +346,8 @@ size_t zkg_batch_kernels(const zkg_batch *batch);
  * Outputs: out_points = 3 G1 XYZZ (32 words each) then 1 G2 XYZZ (64 words); out_h = N elements.
  * Requests queue FIFO; while fewer than `lanes` run, the queue is scanned in order: a request
  * with an idle slot (plans and buffers of its size) starts at once, one without has a slot made
- * for it on a builder thread when that fits the HBM budget (idle slots of other sizes are
+ * for it on a builder thread when that fits the HBM budget (slots give up their affine rounds' scratch,
+ * which they have only while the budget has room for it; then idle slots of other sizes are
  * evicted), and the scan goes on past it; a request whose slot does not fit holds back the ones
  * behind it. Up to `lanes` requests run at once on separate streams, each as one captured CUDA
  * graph with three parallel branches (continuous batching). plain = 1 is the one-call-at-a-time path: one request at a

@@ -196,9 +196,16 @@ size_t MsmPlan::rounds_bytes() const {
   return 4 * words;
 }
 
-void MsmPlan::drop_rounds() {
+void MsmPlan::drop_rounds_locked() {
   rounds = plain;
   release_rounds();  // cudaFree waits for the runs that use it
+}
+
+void MsmPlan::drop_rounds() {
+  spare.unlist();
+  std::lock_guard<std::mutex> lock(queue_mu);
+  drop_rounds_locked();
+  captured = false;
 }
 
 size_t MsmPlan::spare_bytes() const {
@@ -209,7 +216,7 @@ size_t MsmPlan::spare_bytes() const {
 size_t MsmPlan::give_back() {
   std::lock_guard<std::mutex> lock(queue_mu);
   const size_t bytes = captured ? 0 : rounds_bytes();
-  if (bytes) drop_rounds();
+  if (bytes) drop_rounds_locked();
   return bytes;
 }
 

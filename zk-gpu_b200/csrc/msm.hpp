@@ -158,7 +158,7 @@ struct MsmPlan {
   void set_rounds(bool enable);
   uint32_t run_rounds() const { return segments().group_log; }  // of a run as the plan is now
   // Frees the rounds' scratch and goes on without them (queued runs finish first); the rest of the
-  // scratch stays where it is. Called under queue_mu by others than the plan's user.
+  // scratch stays where it is. Graphs captured with the rounds must not be launched any more.
   void drop_rounds();
   size_t rounds_bytes() const;    // of the rounds' scratch
   size_t spare_bytes() const;     // the same, or 0 while a captured graph may hold it
@@ -187,6 +187,7 @@ struct MsmPlan {
   void rank(const uint32_t* bases, const uint32_t* scalars, cudaStream_t s);
   uint32_t item_points_req = 0;
   void release_rounds();
+  void drop_rounds_locked();
 
  public:
   // Held while a run is queued and while the rounds' scratch is given back, by whichever thread.

@@ -11,8 +11,8 @@
 //
 // Slots: the plans and device buffers one request of size class log_m needs, created on demand
 // and reused. Admission: a request leaves the FIFO queue when a free slot of its size exists,
-// or when a new one fits the HBM budget (idle slots of other sizes are evicted to make room)
-// and fewer than `lanes` requests are on the device. Continuous batching: every slot has its
+// or when a new one fits the HBM budget (slots give their affine rounds' scratch and idle slots of
+// other sizes are evicted to make room) and fewer than `lanes` requests are on the device. Continuous batching: every slot has its
 // own stream, so requests admitted while others run overlap on the device; in served mode a
 // request's compute is one CUDA graph, captured when its slot is made, with three parallel
 // branches (G1 MSMs, G2 MSM, NTT chain). Plain mode is the one-call-at-a-time path: one
@@ -109,9 +109,62 @@ const ServerKey* Server::key_for(uint32_t log_m) const {
   return best;
 }
 
-// Whether slots of a size have affine rounds, whose scratch makes a slot of 2^20 points three times as
-// large: where the budget holds twice the slots that may be busy at once, so that no fewer fit.
-bool Server::with_rounds(uint32_t log_m) const { return estimate_bytes(log_m, true) <= budget / (2 * cfg.lanes); }
+// Slots of a size may have affine rounds, whose scratch makes a slot of 2^20 points three times as large,
+// where the budget holds twice the slots that may be busy at once, and those about to be made have them
+// where all of them fit the bytes that are left. What that takes from slots asked for later they get back
+// (ask_rounds), so that the budget holds as many slots as without rounds.
+bool Server::with_rounds(uint32_t log_m, size_t count) const {
+  const size_t need = estimate_bytes(log_m, true);
+  return need <= budget / (2 * cfg.lanes) && bytes_used <= budget && count <= (budget - bytes_used) / need;
+}
+
+// Under mu: marks slots whose rounds' scratch is to go (those already marked, then idle ones, then busy
+// ones) until it adds up to `bytes`, and returns what it adds up to. The dispatcher frees it when the slots
+// are idle (drop_rounds), and bytes_used falls then.
+size_t Server::ask_rounds(size_t bytes) {
+  size_t sum = 0;
+  for (int pass = 0; pass < 3; pass++)
+    for (auto& s : slots) {
+      if (sum >= bytes) return sum;
+      if (!s->rounds_bytes || (s->drop_wanted ? 0 : s->busy ? 2 : 1) != pass) continue;
+      sum += s->rounds_bytes;
+      if (s->drop_wanted) continue;
+      s->drop_wanted = true;
+      cv.notify_all();  // to the dispatcher
+    }
+  return sum;
+}
+
+// Frees the rounds' scratch of slots that the dispatcher has taken (busy), and captures their graphs anew.
+void Server::drop_rounds(const std::vector<ServerSlot*>& dropping) {
+  std::vector<std::unique_ptr<ServerSlot>> lost;
+  for (ServerSlot* s : dropping) {
+    bool whole = true;
+    try {
+      use(ctx);
+      s->g1->drop_rounds();
+      s->g2->drop_rounds();
+      if (s->exec) capture(s);
+    } catch (...) {
+      whole = false;  // without its graph the slot is of no use
+    }
+    std::lock_guard<std::mutex> lock(mu);
+    const size_t freed = whole ? s->rounds_bytes : s->bytes;
+    bytes_used -= std::min(bytes_used, freed);
+    s->bytes -= std::min(s->bytes, freed);
+    s->rounds_bytes = 0;
+    s->drop_wanted = s->busy = false;
+    if (whole) continue;
+    for (size_t i = 0; i < slots.size(); i++)
+      if (slots[i].get() == s) {
+        lost.push_back(std::move(slots[i]));
+        slots.erase(slots.begin() + i);
+        slots_evicted++;
+        break;
+      }
+  }
+  cv.notify_all();
+}
 
 // Device bytes of a slot, from the same formulas the plans allocate with.
 size_t Server::estimate_bytes(uint32_t log_m, bool rounds) const {
@@ -142,7 +195,7 @@ size_t Server::estimate_bytes(uint32_t log_m, bool rounds) const {
 }
 
 
-std::unique_ptr<ServerSlot> Server::make_slot(uint32_t log_m) {
+std::unique_ptr<ServerSlot> Server::make_slot(uint32_t log_m, bool rounds) {
   use(ctx);
   std::unique_ptr<ServerSlot> s(new ServerSlot);
   s->log_m = log_m;
@@ -151,8 +204,8 @@ std::unique_ptr<ServerSlot> Server::make_slot(uint32_t log_m) {
   const size_t m = (size_t)1 << log_m, N = 2 * m;
   size_t free0 = 0, free1 = 0, total = 0;
   check_cuda(cudaMemGetInfo(&free0, &total), "cudaMemGetInfo");
-  s->g1.reset(new MsmPlan(ctx, ZKG_G1, m, default_window(m), 0, with_rounds(log_m)));
-  s->g2.reset(new MsmPlan(ctx, ZKG_G2, m, default_window(m), 0, with_rounds(log_m)));
+  s->g1.reset(new MsmPlan(ctx, ZKG_G1, m, default_window(m), 0, rounds));
+  s->g2.reset(new MsmPlan(ctx, ZKG_G2, m, default_window(m), 0, rounds));
   s->ntt.reset(new NttPlan(ctx, log_m + 1));
   s->shift.reset(new CosetShift(ctx, log_m + 1, cfg.coset_g));
   // 1/g as plain words for the unshift
@@ -173,34 +226,42 @@ std::unique_ptr<ServerSlot> Server::make_slot(uint32_t log_m) {
   for (auto& b : s->branch) check_cuda(cudaStreamCreateWithFlags(&b, cudaStreamNonBlocking), "slot stream");
   check_cuda(cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming), "slot event");
   for (auto& e : s->join) check_cuda(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "slot event");
-  if (!cfg.plain) {
-    // One graph for the request's compute: three branches forked from the slot stream.
-    check_cuda(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "slot capture");
-    try {
-      enqueue_work(s.get(), s->stream, s->branch[0], s->branch[1]);
-    } catch (...) {
-      cudaGraph_t g = nullptr;
-      cudaStreamEndCapture(s->stream, &g);
-      if (g) cudaGraphDestroy(g);
-      cudaGetLastError();
-      throw;
-    }
-    check_cuda(cudaStreamEndCapture(s->stream, &s->graph), "slot capture");
-    check_cuda(cudaGraphInstantiate(&s->exec, s->graph, 0), "slot graph instantiate");
-    size_t nodes = 0;
-    if (cudaGraphGetNodes(s->graph, nullptr, &nodes) == cudaSuccess) {
-      std::vector<cudaGraphNode_t> v(nodes);
-      cudaGraphGetNodes(s->graph, v.data(), &nodes);
-      for (auto nd : v) {
-        cudaGraphNodeType t;
-        if (cudaGraphNodeGetType(nd, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel) s->graph_kernels++;
-      }
-    }
-  }
+  if (!cfg.plain) capture(s.get());
   check_cuda(cudaStreamSynchronize(s->stream), "slot set-up");
   check_cuda(cudaMemGetInfo(&free1, &total), "cudaMemGetInfo");
-  s->bytes = free0 > free1 ? free0 - free1 : estimate_bytes(log_m);
+  s->bytes = free0 > free1 ? free0 - free1 : estimate_bytes(log_m, rounds);
+  s->rounds_bytes = s->g1->rounds_bytes() + s->g2->rounds_bytes();
   return s;
+}
+
+// One graph for the request's compute: three branches forked from the slot stream.
+void Server::capture(ServerSlot* s) {
+  if (s->exec) cudaGraphExecDestroy(s->exec);
+  if (s->graph) cudaGraphDestroy(s->graph);
+  s->exec = nullptr;
+  s->graph = nullptr;
+  s->graph_kernels = 0;
+  check_cuda(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "slot capture");
+  try {
+    enqueue_work(s, s->stream, s->branch[0], s->branch[1]);
+  } catch (...) {
+    cudaGraph_t g = nullptr;
+    cudaStreamEndCapture(s->stream, &g);
+    if (g) cudaGraphDestroy(g);
+    cudaGetLastError();
+    throw;
+  }
+  check_cuda(cudaStreamEndCapture(s->stream, &s->graph), "slot capture");
+  check_cuda(cudaGraphInstantiate(&s->exec, s->graph, 0), "slot graph instantiate");
+  size_t nodes = 0;
+  if (cudaGraphGetNodes(s->graph, nullptr, &nodes) == cudaSuccess) {
+    std::vector<cudaGraphNode_t> v(nodes);
+    cudaGraphGetNodes(s->graph, v.data(), &nodes);
+    for (auto nd : v) {
+      cudaGraphNodeType t;
+      if (cudaGraphNodeGetType(nd, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel) s->graph_kernels++;
+    }
+  }
 }
 
 void Server::enqueue_work(ServerSlot* s, cudaStream_t main, cudaStream_t b0, cudaStream_t b1) {
@@ -282,8 +343,8 @@ void Server::launch(ServerRequest* r, ServerSlot* s) {
 // Admission. The queue is scanned in order while lanes are free: a request with an idle slot of
 // its size is launched at once; one without waits for a busy slot of its size when the size
 // already has max(2, reserved) slots (built or being built), and otherwise gets a slot built for
-// it by the builder thread when the slot fits the HBM budget (after evicting idle slots of other
-// sizes, oldest first); either way the scan goes on, so requests whose slots exist are not held
+// it by the builder thread when the slot fits the HBM budget (after the slots' affine rounds' scratch is
+// freed, and then by evicting idle slots of other sizes, oldest first); either way the scan goes on, so requests whose slots exist are not held
 // up by a slot under construction (measured: a slot built under load took 764 ms, a request of
 // the largest size about 120 ms of kernels).
 // A request whose slot does not fit stops the scan (later requests wait behind it in FIFO order)
@@ -293,6 +354,7 @@ void Server::dispatcher() {
   for (;;) {
     std::vector<std::pair<ServerRequest*, ServerSlot*>> ready;
     std::vector<std::unique_ptr<ServerSlot>> victims;
+    std::vector<ServerSlot*> dropping;
     bool new_builds = false;
     {
       std::unique_lock<std::mutex> lock(mu);
@@ -305,10 +367,11 @@ void Server::dispatcher() {
           const uint32_t log_m = r->desc.log_m;
           ServerSlot* slot = nullptr;
           for (auto& s : slots)
-            if (!s->busy && s->log_m == log_m) {
-              slot = s.get();
-              break;
-            }
+            if (!s->busy && s->log_m == log_m && (!slot || slot->drop_wanted)) slot = s.get();
+          if (slot && slot->drop_wanted) {
+            ++it;  // idle again once its rounds' scratch is gone
+            continue;
+          }
           if (!slot) {
             uint32_t have = building_of[log_m];
             for (auto& s : slots) have += s->log_m == log_m ? 1 : 0;
@@ -317,20 +380,26 @@ void Server::dispatcher() {
               ++it;  // wait for a slot of this size; later requests of other sizes go on
               continue;
             }
-            const size_t need = estimate_bytes(log_m);
-            for (size_t i = 0; i < slots.size() && bytes_used + need > budget;) {
-              if (!slots[i]->busy && slots[i]->log_m != log_m) {
-                bytes_used -= std::min(bytes_used, slots[i]->bytes);
-                victims.push_back(std::move(slots[i]));
-                slots.erase(slots.begin() + i);
-                slots_evicted++;
-              } else {
-                i++;
+            const bool rounds = with_rounds(log_m, 1);
+            const size_t need = estimate_bytes(log_m, rounds);
+            if (bytes_used + need > budget) {
+              // from the other slots' rounds; what those do not make up from idle slots of other sizes
+              size_t coming = ask_rounds(bytes_used + need - budget);
+              for (size_t i = 0; i < slots.size() && bytes_used + need > budget + coming;) {
+                if (!slots[i]->busy && slots[i]->log_m != log_m) {
+                  bytes_used -= std::min(bytes_used, slots[i]->bytes);
+                  if (slots[i]->drop_wanted) coming -= slots[i]->rounds_bytes;
+                  victims.push_back(std::move(slots[i]));
+                  slots.erase(slots.begin() + i);
+                  slots_evicted++;
+                } else {
+                  i++;
+                }
               }
+              if (bytes_used + need > budget && (busy > 0 || coming > 0)) break;  // wait for memory, FIFO from here
             }
-            if (bytes_used + need > budget && busy > 0) break;  // wait for memory, FIFO from here
             bytes_used += need;
-            builds.emplace_back(r, need);
+            builds.push_back(Build{r, need, rounds});
             building++;
             building_of[log_m]++;
             new_builds = true;
@@ -345,12 +414,18 @@ void Server::dispatcher() {
           it = queue.erase(it);
           busy++;
         }
-        if (!ready.empty() || new_builds || !victims.empty()) break;
+        for (auto& s : slots)
+          if (!s->busy && s->drop_wanted) {
+            s->busy = true;
+            dropping.push_back(s.get());
+          }
+        if (!ready.empty() || new_builds || !victims.empty() || !dropping.empty()) break;
         cv.wait(lock);
       }
     }
     if (new_builds) cv.notify_all();
     victims.clear();  // frees device memory outside the lock
+    if (!dropping.empty()) drop_rounds(dropping);
     for (auto& rs : ready) {
       try {
         launch(rs.first, rs.second);
@@ -373,7 +448,7 @@ void Server::dispatcher() {
 void Server::builder() {
   cudaSetDevice(ctx->device);
   for (;;) {
-    std::pair<ServerRequest*, size_t> job;
+    Build job;
     {
       std::unique_lock<std::mutex> lock(mu);
       cv.wait(lock, [&] { return !builds.empty() || (stopping && queue.empty() && building == 0); });
@@ -381,15 +456,15 @@ void Server::builder() {
       job = builds.front();
       builds.pop_front();
     }
-    ServerRequest* r = job.first;
+    ServerRequest* r = job.r;
     ServerSlot* slot = nullptr;
     try {
       const double t0 = now_ms();
-      std::unique_ptr<ServerSlot> s = make_slot(r->desc.log_m);
+      std::unique_ptr<ServerSlot> s = make_slot(r->desc.log_m, job.rounds);
       {
         std::lock_guard<std::mutex> lock(mu);
         build_ms += now_ms() - t0;
-        bytes_used = bytes_used - std::min(bytes_used, job.second) + s->bytes;
+        bytes_used = bytes_used - std::min(bytes_used, job.bytes) + s->bytes;
         slots_created++;
         building--;
         building_of[r->desc.log_m]--;
@@ -404,7 +479,7 @@ void Server::builder() {
       const std::string msg = current_error_text();
       std::lock_guard<std::mutex> lock(mu);
       if (!slot) {
-        bytes_used -= std::min(bytes_used, job.second);
+        bytes_used -= std::min(bytes_used, job.bytes);
         building--;
         building_of[r->desc.log_m]--;
       } else {
@@ -430,22 +505,34 @@ void Server::reserve(uint32_t log_m, uint32_t count) {
   }
   for (;;) {
     size_t need = 0;
+    bool rounds = false;
     {
-      std::lock_guard<std::mutex> lock(mu);
-      uint32_t have = 0;
-      for (auto& s : slots) have += s->log_m == log_m ? 1 : 0;
-      if (have >= count) return;
-      need = estimate_bytes(log_m);
-      if (bytes_used + need > budget)
-        fail(ZKG_ENOMEM, "slot of 2^" + std::to_string(log_m) + " does not fit the HBM budget (" +
-                             std::to_string(budget - std::min(budget, bytes_used)) + " bytes left, " +
-                             std::to_string(need) + " needed)");
+      std::unique_lock<std::mutex> lock(mu);
+      for (;;) {
+        uint32_t have = 0;
+        size_t held = 0;  // by rounds
+        for (auto& s : slots) {
+          have += s->log_m == log_m ? 1 : 0;
+          held += s->rounds_bytes;
+        }
+        if (have >= count) return;
+        rounds = with_rounds(log_m, count - have);
+        need = estimate_bytes(log_m, rounds);
+        if (bytes_used + need <= budget) break;
+        const size_t shortage = bytes_used + need - budget;
+        if (held < shortage && building == 0)  // a slot being made may come to hold some
+          fail(ZKG_ENOMEM, "slot of 2^" + std::to_string(log_m) + " does not fit the HBM budget (" +
+                               std::to_string(budget - std::min(budget, bytes_used)) + " bytes left, " +
+                               std::to_string(need) + " needed)");
+        if (held >= shortage) ask_rounds(shortage);
+        cv.wait(lock);
+      }
       bytes_used += need;
     }
     std::unique_ptr<ServerSlot> s;
     const double t0 = now_ms();
     try {
-      s = make_slot(log_m);
+      s = make_slot(log_m, rounds);
     } catch (...) {
       std::lock_guard<std::mutex> lock(mu);
       bytes_used -= std::min(bytes_used, need);

@@ -29,6 +29,8 @@ struct ServerSlot {
   uint32_t log_m = 0;
   const ServerKey* key = nullptr;
   size_t bytes = 0;
+  size_t rounds_bytes = 0;    // of them, the plans' affine rounds' scratch
+  bool drop_wanted = false;   // the rounds' scratch is to go as soon as the slot is idle
   std::unique_ptr<MsmPlan> g1, g2;
   std::unique_ptr<NttPlan> ntt;
   std::unique_ptr<CosetShift> shift, unshift;
@@ -63,7 +65,12 @@ struct Server {
   std::map<uint64_t, std::unique_ptr<ServerRequest>> requests;
   std::deque<ServerRequest*> queue;
   // admitted requests whose slot is being made, with the bytes reserved for it
-  std::deque<std::pair<ServerRequest*, size_t>> builds;
+  struct Build {
+    ServerRequest* r;
+    size_t bytes;
+    bool rounds;
+  };
+  std::deque<Build> builds;
   int building = 0;  // slots under construction (each holds a lane)
   // Per size: slots reserved by reserve(), slots under construction. A request whose size has
   // max(2, reserved) slots (built or being built), all busy, waits for one of them instead of
@@ -89,10 +96,13 @@ struct Server {
  private:
   void dispatcher();
   void builder();
-  std::unique_ptr<ServerSlot> make_slot(uint32_t log_m);
-  bool with_rounds(uint32_t log_m) const;
+  std::unique_ptr<ServerSlot> make_slot(uint32_t log_m, bool rounds);
+  void capture(ServerSlot* s);
+  // Under mu, of `count` slots about to be made: whether they have affine rounds.
+  bool with_rounds(uint32_t log_m, size_t count) const;
   size_t estimate_bytes(uint32_t log_m, bool rounds) const;
-  size_t estimate_bytes(uint32_t log_m) const { return estimate_bytes(log_m, with_rounds(log_m)); }
+  size_t ask_rounds(size_t bytes);
+  void drop_rounds(const std::vector<ServerSlot*>& dropping);
   const ServerKey* key_for(uint32_t log_m) const;
   void enqueue_work(ServerSlot* s, cudaStream_t main, cudaStream_t b0, cudaStream_t b1);
   void launch(ServerRequest* r, ServerSlot* s);
