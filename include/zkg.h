@@ -113,7 +113,8 @@ int zkg_msm_upload_bases_montgomery_256(zkg_ctx *ctx, const uint32_t *xy, size_t
 
 /* Msm::for_group / new / with_item_points (src/msm.rs:82-180). `c` must be in 9..=20;
  * item_points = 0 picks the work-item size automatically (points accumulated per thread
- * before partial sums are combined). Fails with the reference's messages: "an MSM needs at
+ * before partial sums are combined; in runs with affine rounds, zkg_msm_set_rounds, the points are the
+ * rounds' sums, of 2^rounds entries each). Fails with the reference's messages: "an MSM needs at
  * least one point", "window size c must be in 9..=20, got {c}". */
 int zkg_msm_new(zkg_ctx *ctx, int group, size_t n, uint32_t c, uint32_t item_points, zkg_msm **out);
 void zkg_msm_free(zkg_msm *msm);
@@ -125,7 +126,8 @@ int zkg_msm_group(const zkg_msm *msm);
  * double-precision limbs, products on the FP64 pipe (bit-exact for G1 and G2, slower than the
  * integer forms), 4 = for G1 the plan's own choice, for G2 limbs with one product per call.
  * Defaults: for G1 4, for G2 2.
- * zkg_msm_params reports the plan's window c, points per accumulation thread and form. */
+ * zkg_msm_params reports the plan's window c, points per accumulation thread (as item_points counts
+ * them) and form. */
 int zkg_msm_set_variant(zkg_msm *msm, int variant);
 /* Counting-sort knob (no reference counterpart): how a warp merges the counting pass's atomics
  * for lanes whose digits hit the same (window, bucket) slot: 0 = every group of equal slots,
@@ -287,7 +289,8 @@ int zkg_zkey_upload(zkg_ctx *ctx, const zkg_zkey *zkey, uint32_t section, zkg_bu
 /* ------------------------------------------------------------------ autotuning
  * No reference counterpart (its parameters are fixed: default_window, item size, TILE_LOG).
  * zkg_tune_msm times, on the given inputs, windows c in [default_window(n) - 2, + 2] within
- * 9..=20, 16..256 points per accumulation thread, the accumulation kernel forms and, for G1 with
+ * 9..=20, the plan's own choice (reported as item_points = 0) and 16..256 points per accumulation thread,
+ * the accumulation kernel forms and, for G1 with
  * c <= 16, the GLV split on and off, and writes
  * up to cap results fastest first (out[0] is the choice; *count receives how many).
  * zkg_ntt_set_variant picks a plan's butterfly form: 0 = 32-bit integer products, radix 2 (tiles of

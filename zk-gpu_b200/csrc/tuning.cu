@@ -4,8 +4,8 @@
 // (examples/g2_window.rs:50-69); default_window stays the plain form beside the tuned one.
 //
 // MSM candidates: window c in [default - 2, default + 2] within 9..=20, points per accumulation
-// thread in {16, 32, 64, 128, 256}, the accumulation kernel forms, and for G1 (c <= 16) the GLV
-// split on and off. NTT candidates: the most
+// thread in {the plan's choice, 16, 32, 64, 128, 256}, the accumulation kernel forms, and for G1 (c <= 16)
+// the GLV split on and off. NTT candidates: the most
 // stages per shared-memory pass (passes = ceil(log_n / max_stages)). Each candidate runs once to
 // warm up, then `reps` times between CUDA events; the best mean wins.
 #include <algorithm>
@@ -44,9 +44,10 @@ std::vector<zkg_msm_tuning> tune_msm(zkg_ctx* ctx, int group, size_t n, const zk
     for (int glv = 0; glv <= (group == ZKG_G1 && c <= 16 ? 1 : 0); glv++) {
       const uint32_t windows = glv ? (128 + c - 1) / c : (255 + c - 1) / c;
       const double entries = (double)n * (glv ? 2 : 1) * windows;
-      for (uint32_t L : {16u, 32u, 64u, 128u, 256u}) {
-        // keep at least a few waves of threads on 148 SMs
-        if (entries / L < 148.0 * 256 && L > 16) continue;
+      for (uint32_t L : {0u, 16u, 32u, 64u, 128u, 256u}) {  // 0: the plan's own choice
+        // at least a few waves of threads: of points, which affine rounds make of 2^rounds entries each
+        auto too_few = [&](double points) { return L > 16 && points / L < (double)ctx->sm_count * 256; };
+        if (too_few(entries)) continue;
         std::unique_ptr<MsmPlan> plan;
         try {
           plan.reset(new MsmPlan(ctx, group, n, (uint32_t)c, L));
@@ -60,10 +61,11 @@ std::vector<zkg_msm_tuning> tune_msm(zkg_ctx* ctx, int group, size_t n, const zk
         }
         plan->check_buffers(bases, scalars);
         // out-of-line integer products (1, 2) and, for G1, double-precision limbs (3) and the plan's
-        // own choice (4); form 0 is the same kernel as form 4 for G1 and loses to 1 and 2 for G2
+        // own choice (4); form 0 is form 4 without affine rounds for G1 and loses to 1 and 2 for G2
         const std::vector<int> variants = group == ZKG_G1 ? std::vector<int>{1, 2, 3, 4} : std::vector<int>{1, 2};
         for (int v : variants) {
           plan->acc_variant = v;
+          if (too_few(entries / (1u << plan->run_rounds()))) continue;
           double ms = time_ms(ctx->stream, reps, [&] { plan->enqueue(bases->ptr, scalars->ptr, ctx->stream); });
           out.push_back(zkg_msm_tuning{(uint32_t)c, L, v, glv, ms});
         }

@@ -44,9 +44,9 @@ def _store(cache: dict) -> None:
 
 def search_msm(gpu: Gpu, group: Group, n: int, bases: Buffer, scalars: Buffer, reps: int = 2) -> list[dict]:
     """Every candidate the library timed, fastest first."""
-    arr = (MsmTuning * 128)()
+    arr = (MsmTuning * 256)()
     count = ctypes.c_size_t()
-    check(lib().zkg_tune_msm(gpu.handle, int(group), n, bases.handle, scalars.handle, reps, arr, 128,
+    check(lib().zkg_tune_msm(gpu.handle, int(group), n, bases.handle, scalars.handle, reps, arr, 256,
                              ctypes.byref(count)))
     return [{"c": arr[i].c, "item_points": arr[i].item_points, "variant": arr[i].variant, "glv": arr[i].glv,
              "ms": arr[i].ms} for i in range(count.value)]
