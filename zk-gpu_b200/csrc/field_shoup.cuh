@@ -3,8 +3,10 @@
 // products are needed modulo 2^256 alone.
 //
 // Of the 64 products of words in x w', the 21 below word 6 are left out: together they are under
-// 2^-29 of a unit of q, so q is at most one below the value above and the residue below 3r (below
-// 2.8r for x < 4r). 43 wide multiply-adds there, 28 and eight low halves for each of x w and q r, all on
+// 2^-29 of a unit of q. The real number T that they leave is above x w / r - x / 2^256 - 2^-29 (w' is
+// less than one below w 2^256 / r), and q = floor(T), so the residue is below r (1 + x / 2^256 + 2^-29):
+// below 1.757r for x < 4r, below 2r for x < 2^256 (1 - 2^-29). 43 wide multiply-adds there, 28 and eight
+// low halves for each of x w and q r, all on
 // two interleaved accumulators as in field.cuh: 107 slots of the multiply pipe against the Montgomery
 // product's 132, no chain of digits, and nothing to convert: x w stands in plain form. Measured on
 // B200: 81.3 G products/s, 338 ns for a lone warp (Montgomery: 68.5 G/s, 414 ns).
@@ -207,7 +209,7 @@ __device__ __forceinline__ Fr join_low(const uint32_t (&ev)[8], const uint32_t (
   return r;
 }
 
-// floor(a b / 2^256), or one less (see above).
+// floor of a b / 2^256 less the products below word 6 (see above): that of a b / 2^256, or one less.
 __device__ __forceinline__ void high_product(const uint32_t (&a)[8], const uint32_t (&b)[8], uint32_t (&q)[8]) {
   uint32_t e[10], o[8];  // words 6..15 and 7..14
   mul_pair(e, a[0], b[6]);
@@ -250,7 +252,7 @@ struct Constant {
   Fr w, quotient;
 };
 
-// x c.w modulo r, below 2.8r for x < 4r (below 3r for any x < 2^256).
+// x c.w modulo r, below r (1 + x / 2^256 + 2^-29): below 1.757r for x < 4r.
 __device__ __forceinline__ Fr mul(const Fr& x, const Constant& c) {
   constexpr uint32_t minus_r[8] = {0u - FrParams::P0, ~FrParams::P1, ~FrParams::P2, ~FrParams::P3,
                                    ~FrParams::P4,     ~FrParams::P5, ~FrParams::P6, ~FrParams::P7};

@@ -11,8 +11,9 @@
 // pass; the rest goes to the tiles' loads and stores, which other blocks' products cover in part.
 //
 // Bounds: r < 0.19 2^256, so 5r < 2^256. Elements between steps are below 2r; a sum of two is
-// brought below 2r again by one conditional subtraction of 2r, and so is a product (below 2.8r); a
-// difference gets 2r added and is a product's operand (below 4r).
+// brought below 2r again by one conditional subtraction of 2r; a difference gets 2r added and is a
+// product's operand (below 4r), and the product by a twiddle is below 1.757r (field_shoup.cuh): the
+// conditional subtraction that follows it too (`times`) finds nothing to take off.
 #pragma once
 #include "field_shoup.cuh"
 
