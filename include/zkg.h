@@ -456,6 +456,13 @@ int zkg_bench_integer_pipe(zkg_ctx *ctx, int variant, double *ops_per_second);
  * three XYZZ points: P + Q (mixed add), 2P (double), (P + Q) + 2P (full add). */
 int zkg_test_point_ops(zkg_ctx *ctx, int group, const uint32_t *pairs, size_t count, uint32_t *out);
 
+/* Field operations that the point formulas above do not run, of `count` items in host memory (Montgomery words,
+ * fully reduced unless said otherwise): op 0, Fq2 products with one reduction per component (the G2 kernels'
+ * form): x, y, z, w -> x y, x^2, x y - z w; op 1 and 2, 1/x in Fq and Fq2 (zero for zero); op 3, a
+ * product by a constant of Fr with its quotient: x (any 8 words), the constant's Montgomery form ->
+ * a residue of their plain product, the plain constant, floor(constant 2^256 / r). */
+int zkg_test_field_ops(zkg_ctx *ctx, int op, const uint32_t *in, size_t count, uint32_t *out);
+
 /* The device's GLV split (zkg_msm_set_glv) of `count` scalars in host memory (8 words each):
  * out[10 i ..] = |k1| (4 words), |k2| (4 words), sign of k1, sign of k2 (1 = negative), with k =
  * k1 + k2 lambda (mod r), lambda = 0x30644e72e131a029048b6e193fd84104cc37a73fec2bc5e9b8ca0b2d36636f23. */

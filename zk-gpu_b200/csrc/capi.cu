@@ -1012,6 +1012,16 @@ int zkg_test_point_ops(zkg_ctx* ctx, int group, const uint32_t* pairs, size_t co
   });
 }
 
+int zkg_test_field_ops(zkg_ctx* ctx, int op, const uint32_t* in, size_t count, uint32_t* out) {
+  return guard([&] {
+    need(ctx, "ctx");
+    need(in, "in");
+    need(out, "out");
+    if (!field_op_words(op, false)) fail(ZKG_EINVAL, "field operation must be 0..3");
+    if (count) field_ops(ctx, op, in, count, out);
+  });
+}
+
 int zkg_generator_multiples(zkg_ctx* ctx, int group, const zkg_buf* scalars, size_t n, int mont256, zkg_buf* out) {
   return guard([&] {
     need(ctx, "ctx");

@@ -175,4 +175,26 @@ __device__ __noinline__ Fp<P> mont_inverse(Fp<P> a, Fp<P> r3) {
   return mont_mul_prod(r, r3);
 }
 
+// 1/a in Montgomery form of the base field's forms (zero for zero).
+template <class P>
+__device__ __forceinline__ Fp<P> affine_inverse(const Fp<P>& a) {
+  Fp<FqParams> x, r3;
+#pragma unroll
+  for (int i = 0; i < 8; i++) {
+    x.w[i] = a.w[i];
+    r3.w[i] = kFqR3[i];
+  }
+  const Fp<FqParams> y = mont_inverse<FqParams>(x, r3);
+  Fp<P> r;
+#pragma unroll
+  for (int i = 0; i < 8; i++) r.w[i] = y.w[i];
+  return r;
+}
+// 1 / (a + bu) = (a - bu) / (a^2 + b^2)
+template <class B>
+__device__ __forceinline__ Fq2T<B> affine_inverse(const Fq2T<B>& x) {
+  const B inv = affine_inverse(sqr(x.a) + sqr(x.b));
+  return Fq2T<B>{x.a * inv, neg(x.b * inv)};
+}
+
 }  // namespace zkg

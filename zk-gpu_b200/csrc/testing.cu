@@ -5,6 +5,8 @@
 
 #include "curve.cuh"
 #include "field_f64.cuh"
+#include "field_inverse.cuh"
+#include "field_shoup.cuh"
 #include "host_field.hpp"
 #include "runtime.hpp"
 #include "testing.hpp"
@@ -50,6 +52,54 @@ void point_ops(zkg_ctx* ctx, int group, const uint32_t* pairs, size_t count, uin
   check_launch("point_ops_kernel");
   check_cuda(cudaMemcpyAsync(out, res.ptr, count * 12 * w * 4, cudaMemcpyDeviceToHost, ctx->stream), "copy");
   check_cuda(cudaStreamSynchronize(ctx->stream), "point ops");
+}
+
+// ------------------------------------------------------------------ field ops test
+
+template <int OP>
+__global__ void field_ops_kernel(const uint32_t* __restrict__ in, size_t count, size_t in_words, size_t out_words,
+                                 uint32_t* __restrict__ out) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= count) return;
+  const uint32_t* p = in + i * in_words;
+  uint32_t* o = out + i * out_words;
+  if constexpr (OP == 0) {
+    const Fq2L x = load_elem<Fq2L>(p), y = load_elem<Fq2L>(p + 16), z = load_elem<Fq2L>(p + 32), w = load_elem<Fq2L>(p + 48);
+    store_elem(o, x * y);
+    store_elem(o + 16, sqr(x));
+    store_elem(o + 32, mul_sub(x, y, z, w));
+  } else if constexpr (OP == 1) {
+    store_elem(o, affine_inverse(load_elem<Fq>(p)));
+  } else if constexpr (OP == 2) {
+    store_elem(o, affine_inverse(load_elem<Fq2L>(p)));
+  } else {
+    const shoup::Constant c = shoup::constant(load_fe<Fr>(p + 8));
+    store_fe(o, shoup::mul(load_fe<Fr>(p), c));
+    store_fe(o + 8, c.w);
+    store_fe(o + 16, c.quotient);
+  }
+}
+
+size_t field_op_words(int op, bool results) {
+  constexpr size_t words[4][2] = {{64, 48}, {8, 8}, {16, 16}, {16, 24}};
+  return op < 0 || op > 3 ? 0 : words[op][results];
+}
+
+void field_ops(zkg_ctx* ctx, int op, const uint32_t* in, size_t count, uint32_t* out) {
+  use(ctx);
+  const size_t iw = field_op_words(op, false), ow = field_op_words(op, true);
+  DeviceArray src, res;
+  src.alloc(count * iw, "field ops input");
+  res.alloc(count * ow, "field ops output");
+  check_cuda(cudaMemcpyAsync(src.ptr, in, count * iw * 4, cudaMemcpyHostToDevice, ctx->stream), "copy");
+  auto launch = [&](auto kernel) { kernel<<<grid_for(count, 64), 64, 0, ctx->stream>>>(src.ptr, count, iw, ow, res.ptr); };
+  if (op == 0) launch(field_ops_kernel<0>);
+  else if (op == 1) launch(field_ops_kernel<1>);
+  else if (op == 2) launch(field_ops_kernel<2>);
+  else launch(field_ops_kernel<3>);
+  check_launch("field_ops_kernel");
+  check_cuda(cudaMemcpyAsync(out, res.ptr, count * ow * 4, cudaMemcpyDeviceToHost, ctx->stream), "copy");
+  check_cuda(cudaStreamSynchronize(ctx->stream), "field ops");
 }
 
 // ------------------------------------------------------------------ generator multiples

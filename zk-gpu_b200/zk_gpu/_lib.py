@@ -142,6 +142,7 @@ SIGNATURES = {
                                           ctypes.POINTER(ctypes.c_size_t), ctypes.POINTER(ctypes.c_size_t)]),
     "zkg_bench_integer_pipe": (ctypes.c_int, [vp, ctypes.c_int, ctypes.POINTER(ctypes.c_double)]),
     "zkg_test_point_ops": (ctypes.c_int, [vp, ctypes.c_int, u32p, ctypes.c_size_t, u32p]),
+    "zkg_test_field_ops": (ctypes.c_int, [vp, ctypes.c_int, u32p, ctypes.c_size_t, u32p]),
     "zkg_test_glv_split": (ctypes.c_int, [vp, u32p, ctypes.c_size_t, u32p]),
     "zkg_generator_multiples": (ctypes.c_int, [vp, ctypes.c_int, vp, ctypes.c_size_t, ctypes.c_int, vp]),
 }
