@@ -539,8 +539,13 @@ void MsmPlan::stage(int which, const uint32_t* bases, const uint32_t* scalars, c
         // a warp for each pair of windows (msm_combine_lanes)
         using A = typename std::conditional<std::is_same<F, Fq>::value, Fq, typename CompactOf<F>::type>::type;
         const uint32_t width = glv ? 128u / windows : c, extra = glv ? 128u % windows : 0u;
-        msm_combine_lanes<A><<<1, 32 * std::max(1u, active_windows() / 2), 0, s>>>(window_sums.ptr, active_windows(), width,
-                                                                                    extra, combine_out);
+        const uint32_t warps = std::max(1u, active_windows() / 2);
+        auto launch = [&](auto kernel) {
+          kernel<<<1, 32 * warps, 0, s>>>(window_sums.ptr, active_windows(), width, extra, combine_out);
+        };
+        constexpr uint32_t few = CombineWarps<A>::value;
+        if (warps <= few) launch(msm_combine_lanes<A, few>);
+        else launch(msm_combine_lanes<A, kCombineWindows / 2>);
       }
       check_launch("msm_combine_lanes");
       if (!first_pass) {  // a later pass: add its point into the result

@@ -1089,9 +1089,17 @@ __global__ void __launch_bounds__(kFoldValues / 2 * 32)
 // for the plain windows, the glv_window_width split for GLV. Bound by the latency of the doublings'
 // products; one chain (Horner) took W - 1 additions, 5.7 us each with their start of a chain (G2
 // 8.9): G1 of 12 windows 0.169 ms, now 0.155, G2 of 24 0.495, now 0.440.
+// WARPS bounds the block, and with it the registers. An Fq2 chain wants more than the 128 that 16 warps
+// leave (192 bytes of spills stored, 76 loaded); bound to the 12 that the default windows take, it has 168
+// and reloads nothing: G2 2^14 1076 us, 1080 before. G1 takes 88 of the 128, and bound to 12 its schedule is
+// the slower (G1 of 1000 points 386 us against 383.4), so it keeps one form.
 constexpr uint32_t kCombineWindows = 32;  // 255 bits in windows of 9, at most
 template <class F>
-__global__ void __launch_bounds__(kCombineWindows / 2 * 32)
+struct CombineWarps {
+  static constexpr uint32_t value = PointWords<F>::xyzz == 32 ? kCombineWindows / 2 : 12;
+};
+template <class F, uint32_t WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
     msm_combine_lanes(const uint32_t* __restrict__ window_sums, uint32_t windows, uint32_t base, uint32_t extra,
                       uint32_t* __restrict__ result) {
   constexpr int XW = PointWords<F>::xyzz;
