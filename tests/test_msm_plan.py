@@ -117,6 +117,31 @@ def test_rounds_switched_off_and_on(gpu):
     assert msm.rounds() == (0, scratch) and run() == want
 
 
+def test_a_change_that_does_not_fit_leaves_an_error(gpu):
+    """A slice whose scratch the device has no room for is refused, and so are runs (the plan has lost the
+    scratch of before, not only part of it) until a slice that fits."""
+    from zk_gpu import ZkGpuError
+    n = 1 << 22
+    bases = generator_multiples(gpu, Group.G1, uniform_scalars(n, 3), mont256=True)
+    scalars = gpu.buffer(uniform_scalars(n, 4))
+    msm = Msm(gpu, n, Msm.default_window(n))
+    msm.set_chunk(1 << 16)
+    run = lambda: xyzz_to_affine(gpu.read(msm.run(gpu, bases, scalars), 32))  # noqa: E731
+    want = run()
+    ballast = gpu.empty_buffer((free_bytes() - (GIB >> 2)) // 4)
+    with pytest.raises(ZkGpuError, match="out of memory"):
+        msm.set_chunk(n)
+    with pytest.raises(ZkGpuError, match="no scratch"):
+        run()
+    with pytest.raises(ZkGpuError, match="no scratch"):
+        msm.profile(gpu, bases, scalars)
+    msm.set_chunk(1 << 16)
+    assert run() == want
+    ballast.free()
+    msm.set_chunk(0)
+    assert run() == want
+
+
 def test_scratch_given_back_while_another_thread_runs_the_plan(gpu):
     """One thread runs the plan over and over, another one's allocation takes the rounds' scratch."""
     msm, bases, scalars, run = large(gpu)

@@ -137,7 +137,7 @@ void MsmPlan::set_chunk(size_t points) {
   use(ctx);
   chunk_req = points;
   const size_t want = std::min(n, std::min(points ? points : n, max_chunk()));
-  if (want != chunk) {
+  if (want != chunk || !laid_out) {
     chunk = want;
     layout();
   }
@@ -229,7 +229,7 @@ void MsmPlan::set_rounds(bool enable) {
 // Where the affine rounds' scratch does not fit the device beside the rest, the plan goes without.
 void MsmPlan::layout() {
   spare.unlist();
-  captured = false;
+  captured = laid_out = false;
   release_rounds();
   const size_t np = glv ? 2 * chunk : chunk;
   windows = glv ? (128 + c - 1) / c : (255 + c - 1) / c;
@@ -243,6 +243,7 @@ void MsmPlan::layout() {
       return;
     } catch (const Error& e) {
       if (e.code != ZKG_ENOMEM) throw;
+      laid_out = true;
       release_rounds();
     }
   }
@@ -251,6 +252,12 @@ void MsmPlan::layout() {
 
 void MsmPlan::layout_rounds(uint32_t group_log) {
   const size_t np = glv ? 2 * chunk : chunk;  // points of the largest pass
+  laid_out = true;
+}
+
+void MsmPlan::check_laid_out() const {
+  if (!laid_out)
+    fail(ZKG_ENOMEM, "the MSM plan has no scratch: its last change of layout ran out of device memory");
   const size_t xw = xyzz_words();
   const size_t max_entries = (size_t)windows * np;
   const size_t tile = group == ZKG_G1 ? MergeTile<FqCP>::value : MergeTile<Fq2L>::value;
@@ -372,7 +379,7 @@ bool MsmPlan::glv_default() const {
 }
 
 void MsmPlan::set_glv(bool enable) {
-  if (enable == glv) return;
+  if (enable == glv && laid_out) return;
   if (enable) {
     if (group != ZKG_G1) fail(ZKG_EINVAL, "GLV splitting is for G1 (the endomorphism (x, y) -> (beta x, y))");
     if (c > 16) fail(ZKG_EINVAL, "GLV splitting needs a window size c <= 16, got " + std::to_string(c));
@@ -399,7 +406,7 @@ void MsmPlan::set_fixed_base(bool enable) {
   if (enable && plain_windows * n >= (size_t)kNegBit)
     fail(ZKG_EINVAL, "a fixed-base table holds fewer than 2^31 points");
   if (enable && glv) set_glv(false);  // the table's rows are the plain windows
-  if (enable && chunk != n) {  // one pass: the table's rows are n points apart
+  if (enable && (chunk != n || !laid_out)) {  // one pass: the table's rows are n points apart
     chunk = n;
     layout();
   }
@@ -688,6 +695,7 @@ void MsmPlan::enqueue(const uint32_t* bases, const uint32_t* scalars, cudaStream
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     check_cuda(cudaStreamIsCapturing(s, &status), "stream capture status");
     captured = status != cudaStreamCaptureStatusNone;
+  check_laid_out();
   }
   for (size_t off = 0; off < n; off += chunk) {
     const uint32_t *b = bases, *sc = scalars;
@@ -716,6 +724,7 @@ std::vector<std::pair<std::string, double>> MsmPlan::profile(const zkg_buf* base
   cudaEvent_t a, b;
   check_cuda(cudaEventCreate(&a), "event");
   check_cuda(cudaEventCreate(&b), "event");
+  check_laid_out();
   for (int st = 0; st < kStages; st++) out.emplace_back(stage_name(st), 0.0);
   for (size_t off = 0; off < n; off += chunk) {  // stage times summed over the passes
     const uint32_t *bp = bases->ptr, *sp = scalars->ptr;

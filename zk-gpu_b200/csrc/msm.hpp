@@ -188,6 +188,10 @@ struct MsmPlan {
   uint32_t item_points_req = 0;
   void release_rounds();
   void drop_rounds_locked();
+  // Every array of the scratch is there; not after a change of layout that ran out of memory, until one
+  // that fits.
+  bool laid_out = false;
+  void check_laid_out() const;
 
  public:
   // Held while a run is queued and while the rounds' scratch is given back, by whichever thread.
