@@ -8,7 +8,7 @@
 // each computes one of the four products, for chains with nothing beside them to fill the warp. Values
 // pass between roles by shuffles within the group; every lane of a warp takes part in every call.
 //
-// A lone warp's product takes 414 ns, a b - c d 611 ns; measured on B200 per doubling in the chain of
+// A lone warp's product takes 428 ns, a b - c d 611 ns; measured on B200 per doubling in the chain of
 // the window combination (LaneChain), G1 1.1 us, G2 1.65 (dbl-2008-s-1, three products deep: 1.6 and
 // 2.4; two lanes a role: G2 2.65). Every lane used to hold the whole point and to form every level's
 // sums itself through shared memory: 1.9 and 5.4 us.
@@ -21,19 +21,15 @@ template <class F, int SPLIT = 1>
 struct LaneGroup;
 template <class P, int SPLIT>
 struct LaneGroup<Fp<P>, SPLIT> {  // a product of Fq is not split
-  static constexpr unsigned kLanes = 8, kComponents = 1, kPerRole = 1;
+  static constexpr unsigned kLanes = 8, kPerRole = 1;
 };
 template <class B, int SPLIT>
 struct LaneGroup<Fq2T<B>, SPLIT> {
-  static constexpr unsigned kLanes = 16 * SPLIT, kComponents = 2, kPerRole = 2 * SPLIT;
+  static constexpr unsigned kLanes = 16 * SPLIT, kPerRole = 2 * SPLIT;
 };
 template <class F, int SPLIT = 1>
 __device__ __forceinline__ unsigned lane_role() {
   return (threadIdx.x & (LaneGroup<F, SPLIT>::kLanes - 1)) / LaneGroup<F, SPLIT>::kPerRole;
-}
-template <class F>
-__device__ __forceinline__ unsigned lane_component() {
-  return threadIdx.x & (LaneGroup<F>::kComponents - 1);
 }
 
 // The value a role of this group holds (role: may differ between lanes).

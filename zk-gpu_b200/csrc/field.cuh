@@ -5,8 +5,9 @@
 //
 // Replaces the reference's generated WGSL field code (src/field.rs:55-181: 20 x 13-bit limbs,
 // R = 2^260, deferred carries). Memory format is unchanged: 8 little-endian u32 words per
-// element (src/field.rs:63-93). Values in registers and in memory are always fully reduced
-// (< p), so equality and zero tests are word compares.
+// element (src/field.rs:63-93). Values in memory, and those that are compared, are fully reduced
+// (< p), so equality and zero tests are word compares; operands that a function takes or leaves
+// unreduced have their bounds stated at it.
 #pragma once
 #include <cstdint>
 
@@ -179,7 +180,8 @@ __device__ __forceinline__ Fp<P> dbl(const Fp<P>& a) {
 
 // ------------------------------------------------------------------ Montgomery product
 //
-// Operand scanning with 32x32 -> 64-bit products held as two interleaved accumulators: `e` sums
+// Operand scanning (Koc, Acar and Kaliski, "Analyzing and comparing Montgomery multiplication
+// algorithms", 1996) with 32x32 -> 64-bit products held as two interleaved accumulators: `e` sums
 // the products whose low word falls on an even position and `o` those on an odd one, so every
 // product is added to an aligned pair of words and consecutive products of one accumulator
 // continue each other's carry chain. A mad.lo.cc / madc.hi.cc pair on such a pair of words is one
@@ -187,8 +189,8 @@ __device__ __forceinline__ Fp<P> dbl(const Fp<P>& a) {
 // add.cc over their halves) needed about 450 warp instructions per product, this one about 190:
 // 128 wide multiply-adds, 8 multiples m = t_0 INV and the carries. The wide multiply-add issues at
 // half rate, so 132 full-rate slots of that pipe bound it. Measured on B200: 68 G products/s (the
-// pipe's limit) from two warps per scheduler on, 425 ns for a lone warp; before, 49.8 G/s and
-// 518 ns.
+// pipe's limit) from two warps per scheduler on, 428 ns for a lone warp (422 before the last
+// subtraction of p); before, 49.8 G/s and 518 ns.
 //
 // After the multiply row and the reduction row of word i, word 0 is zero and the value moves one
 // word down: `o` becomes the even accumulator, and e[1] is added into its word 0 with the carry
@@ -394,7 +396,7 @@ __device__ __forceinline__ void sqr_chain(uint32_t* c, const uint32_t (&x)[N], u
 
 // a^2 2^-256 mod p up to one p (a < 2^255): 36 products of words (each cross product once, with one
 // factor doubled) and the reduction rows over the low half, 100 wide multiply-adds against 128:
-// 78.6 G/s, 345 ns for a lone warp (product: 68.1 G/s, 414 ns).
+// 78.6 G/s, 356 ns for a lone warp (product: 68.1 G/s, 422 ns).
 template <class P>
 __device__ __forceinline__ Fp<P> mont_sqr_lazy(const Fp<P>& a) {
   const uint32_t* w = a.w;

@@ -4,7 +4,8 @@
 // Replaces the reference's host bignum (src/host.rs:1-115: U256 add/sub/mul/pow/inverse,
 // root_of_unity with generator 5, words32 packing) and xyzz_to_affine(_g2) with its Fq2
 // helpers (src/msm.rs:345-387). Montgomery radix here is 2^256, matching the device code.
-// Never on the hot path: used a few thousand times per plan at most.
+// Runs at plan set-up (a few thousand products), and once per result that a caller converts to
+// affine coordinates: two inversions, 24-28 us a point on the host.
 #pragma once
 #include <cstdint>
 #include <cstring>

@@ -84,7 +84,11 @@ static uint32_t affine_per_thread(size_t pairs, int group, int sms) {
 // 1.01 / 1.44, 2^18 2.78 / 2.30 / 2.60 / 3.63, 2^20 8.73 / 7.12 / 7.90 / 11.5, 2^22 32.3 / 28.1 / 27.1. The
 // entries are the most there can be: sparse scalars (three in five zero digits) gain from larger sizes
 // on than uniform ones, so the line lies at 2^19 and G2 2^18 points (a sparse G1 MSM of 300007 points:
-// 1.01 ms without rounds, 1.09 with two).
+// 1.01 ms without rounds, 1.09 with two). There they lose little yet: whole MSMs, ms, without / with two
+// rounds, uniform and sparse: G1 2^19 2.35 / 2.18 and 1.44 / 1.47, 2^20 3.73 / 3.32 and 2.26 / 2.08; G2 2^18
+// 3.95 / 3.47 and 2.50 / 2.63, 2^19 6.57 / 5.76 and 4.04 / 3.89. A fixed-base plan is laid out by the slots of
+// all windows although its runs fill one set: G1 2^19 2.27 / 2.18 and 1.37 / 1.46, 2^20 3.43 / 3.31 and 2.03 /
+// 2.05.
 uint32_t MsmPlan::affine_rounds(size_t entries) const {
   if (!affine) return 0;
   const size_t per_slot = entries / slots;
@@ -239,25 +243,25 @@ void MsmPlan::layout() {
   if (const uint32_t group_log = affine_rounds(windows * np)) {
     try {
       layout_rounds(group_log);
+      laid_out = true;
       spare.list(this);
       return;
     } catch (const Error& e) {
       if (e.code != ZKG_ENOMEM) throw;
-      laid_out = true;
       release_rounds();
     }
   }
   layout_rounds(0);
-}
-
-void MsmPlan::layout_rounds(uint32_t group_log) {
-  const size_t np = glv ? 2 * chunk : chunk;  // points of the largest pass
   laid_out = true;
 }
 
 void MsmPlan::check_laid_out() const {
   if (!laid_out)
     fail(ZKG_ENOMEM, "the MSM plan has no scratch: its last change of layout ran out of device memory");
+}
+
+void MsmPlan::layout_rounds(uint32_t group_log) {
+  const size_t np = glv ? 2 * chunk : chunk;  // points of the largest pass
   const size_t xw = xyzz_words();
   const size_t max_entries = (size_t)windows * np;
   const size_t tile = group == ZKG_G1 ? MergeTile<FqCP>::value : MergeTile<Fq2L>::value;
@@ -371,8 +375,8 @@ void MsmPlan::check_buffers(const zkg_buf* bases, const zkg_buf* scalars) const 
 }
 
 // GLV is the G1 default wherever it applies: measured faster than the plain windows at every
-// default window on B200 (2^16: 1.35 against 1.69 ms; 2^18: 2.31 / 2.76; 2^20: 5.53 / 5.83;
-// 2^22: 15.7 / 16.7; 2^24: 54.8 / 55.1), half the reduction and combination work for the same
+// default window on B200 (2^16: 0.70 against 0.87 ms; 2^18: 1.38 / 1.57; 2^20: 3.32 / 3.46;
+// 2^22: 10.3 / 10.7; 2^24: 39.2 / 39.7), half the reduction and combination work for the same
 // bucket additions.
 bool MsmPlan::glv_default() const {
   return group == ZKG_G1 && c <= 16;
@@ -691,11 +695,11 @@ void MsmPlan::begin_pass(size_t off, const uint32_t*& bases, const uint32_t*& sc
 
 void MsmPlan::enqueue(const uint32_t* bases, const uint32_t* scalars, cudaStream_t s) {
   std::lock_guard<std::mutex> lock(queue_mu);
+  check_laid_out();
   if (segments().group_log && !captured) {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     check_cuda(cudaStreamIsCapturing(s, &status), "stream capture status");
     captured = status != cudaStreamCaptureStatusNone;
-  check_laid_out();
   }
   for (size_t off = 0; off < n; off += chunk) {
     const uint32_t *b = bases, *sc = scalars;
@@ -720,11 +724,11 @@ std::vector<std::pair<std::string, double>> MsmPlan::profile(const zkg_buf* base
   check_buffers(bases, scalars);
   use(ctx);
   std::lock_guard<std::mutex> lock(queue_mu);
+  check_laid_out();
   std::vector<std::pair<std::string, double>> out;
   cudaEvent_t a, b;
   check_cuda(cudaEventCreate(&a), "event");
   check_cuda(cudaEventCreate(&b), "event");
-  check_laid_out();
   for (int st = 0; st < kStages; st++) out.emplace_back(stage_name(st), 0.0);
   for (size_t off = 0; off < n; off += chunk) {  // stage times summed over the passes
     const uint32_t *bp = bases->ptr, *sp = scalars->ptr;

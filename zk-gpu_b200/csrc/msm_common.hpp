@@ -8,8 +8,7 @@ namespace zkg {
 constexpr uint32_t kNegBit = 0x80000000u;
 constexpr uint32_t kNoKey = 0xffffffffu;
 constexpr uint32_t kPadEntry = 0xffffffffu;  // a place of the sorted array without an entry (infinity)
-// Heads summed per thread per merge level, and buckets per running-sum thread (2^chunk_log),
-// chosen per plan: long chains suit many threads, short ones few (MsmPlan).
+// The scan over the slots: threads of a block, values of a thread.
 constexpr int kScanBlock = 1024;
 constexpr int kScanItems = 4;
 constexpr int kScanTile = kScanBlock * kScanItems;

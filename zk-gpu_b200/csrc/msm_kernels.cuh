@@ -25,7 +25,8 @@
 //                       second sum is the same problem over run_1.. [msm_reduce_chunks.wgsl]
 //   7. window sums      per window the last vector's columns and rows, their bits' sums, and the
 //                       fold of those by doublings                [msm_sum.wgsl]
-//   8. combine          Horner over windows, c doublings each      [msm_combine.wgsl]
+//   8. combine          neighbouring windows pairwise, each pair's upper one doubled by the width of
+//                       the lower                                  [msm_combine.wgsl]
 #pragma once
 #include "curve.cuh"
 #include "curve_lanes.cuh"
@@ -678,13 +679,6 @@ __device__ __forceinline__ uint32_t last_leq(const uint32_t* a, uint32_t lo, uin
   return lo;
 }
 
-template <class F>
-__device__ __forceinline__ Affine<F> load_signed_base(const uint32_t* __restrict__ bases, uint32_t entry) {
-  Affine<F> p = load_affine<F>(bases + (size_t)(entry & ~kNegBit) * PointWords<F>::affine);
-  if (entry & kNegBit) p.y = neg(p.y);
-  return p;
-}
-
 // One thread per segment [t*L, t*L + L) of the sorted entries (all windows concatenated, slot
 // order). slot_start has num_slots + 1 entries; slot_start[num_slots] = total entries.
 // Points below `split` come from `bases`, the others from bases2 (point - split): the GLV
@@ -929,9 +923,9 @@ __global__ void __launch_bounds__(kReduceThreads) msm_reduce_level(const uint32_
 // The last level: S = sum_i (i + 1) A_i over m <= kMarginalMax values per window, by marginals. With i =
 // l + 2^lo h, sum_i i A_i = sum_l l C_l + 2^lo sum_h h R_h, C_l the sum of column l and R_h of row h; and
 // over the bits of l, sum_l l C_l = sum_k 2^k Z_k, Z_k the sum of the C_l whose l has bit k, likewise for
-// h. So three launches: the columns and rows (each at most 64 values), the Z_k and sum_l C_l (at most 32
-// columns or rows each), and the fold. All are trees, about log2(64) + log2(32) additions deep where
-// running sums and a suffix scan over 256 threads made 26 additions, on one SM per window.
+// h. So three launches: the columns and rows (each at most 64 values), the Z_k (at most 32 columns or
+// rows each) and sum_l C_l (at most 64 columns), and the fold. All are trees, at most 2 log2(64) additions
+// deep where running sums and a suffix scan over 256 threads made 26 additions, on one SM per window.
 //
 // A sum of points that a block forms: which values of a window's vector, and how many.
 enum SubsetKind : uint32_t { kColumn, kRow, kBit, kAll };
@@ -961,7 +955,8 @@ struct Subset {
 };
 
 // *out = the sum over the subset of the window's vector at `in`; a value whose slot is empty
-// (slot_start, when given, has the window's slots) is the point at infinity. One block.
+// (slot_start, when given, has the window's slots) is the point at infinity. One block of at least
+// PointWords<F>::xyzz threads.
 template <class F>
 __device__ __forceinline__ void subset_sum(const Subset& s, const uint32_t* __restrict__ in,
                                            const uint32_t* __restrict__ slot_start, uint32_t* __restrict__ out,
@@ -982,7 +977,6 @@ __device__ __forceinline__ void subset_sum(const Subset& s, const uint32_t* __re
   __syncthreads();
   tree_sum<F>(sh, n);
   if (threadIdx.x < XW) out[threadIdx.x] = sh[threadIdx.x];
-  if (XW > blockDim.x && threadIdx.x + blockDim.x < XW) out[threadIdx.x + blockDim.x] = sh[threadIdx.x + blockDim.x];
 }
 
 // Threads of a subset's block: one warp for G1 (a window has at least 64 subsets), four for G2, whose
