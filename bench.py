@@ -40,10 +40,10 @@ IMAD_PER_MULMOD = 264  # 8 rows x (16 product + 16 reduction multiply-adds + 1 m
 MULMODS_PER_MADD = 10  # madd-2008-s: 8M + 2S
 MULMODS_PER_AFFINE = 6  # an affine addition with a shared inversion: 5M + 1S (msm_affine.cuh)
 # ncu DRAM traffic (read + write bytes), default plans. Accumulation: the launches of its affine rounds
-# and msm_accumulate on a G1 MSM of 2^22 points, scaled by the entry count to 2^24 (x4); NTT: per
-# launch, forms 0, 1 and 2 the first pass on the 2^24 transform.
+# (three) and msm_accumulate on a G1 MSM of 2^22 points, the size that was measured; NTT: per launch,
+# forms 0, 1 and 2 the first pass on the 2^24 transform.
 NCU_TRAFFIC = {
-    "msm_accumulate_2^24": 118.4e9,
+    "msm_accumulate_2^22": 29.6e9,
     "ntt_form0_2^24": 1.96e9,
     "ntt_form1_2^24": 2.18e9,
     "ntt_form2_2^24": 2.12e9,
@@ -346,9 +346,7 @@ def run_ours(a, d: Dist) -> dict | None:
 
     # ---- rooflines
     acc_ms = st24.get("accumulate", float("nan"))
-    # the plan's affine rounds halve what is left for mixed additions each (MsmPlan::affine_rounds)
-    most = (1 << a.log_msm) * 2 * -(-128 // c24)
-    rounds = 4 if most >= 1 << 28 else 3 if most >= 1 << 26 else 2 if most >= 1 << 23 else 0
+    rounds = msm24.rounds()[0]  # each halves what is left for mixed additions
     mulmods_per_entry = MULMODS_PER_AFFINE * (1 - 2.0 ** -rounds) + MULMODS_PER_MADD * 2.0 ** -rounds
     acc_ops = entries.value * mulmods_per_entry * IMAD_PER_MULMOD
     acc_achieved = acc_ops / (acc_ms * 1e-3)
@@ -399,7 +397,8 @@ def run_ours(a, d: Dist) -> dict | None:
             "peak": round(imad_peak / 1e12, 3),
             "unit": "T int-mul-add/s",
             "frac": round(acc_achieved / imad_peak, 4),
-            "traffic": NCU_TRAFFIC["msm_accumulate_2^24"],
+            "traffic": NCU_TRAFFIC.get(f"msm_accumulate_2^{a.log_msm}"),
+            "traffic_2^22": NCU_TRAFFIC["msm_accumulate_2^22"],
             "algorithmic": f"{entries.value} nonzero digits x {mulmods_per_entry} Fq products ({MULMODS_PER_AFFINE} an "
                            f"affine, {MULMODS_PER_MADD} a mixed addition) x {IMAD_PER_MULMOD} 32-bit multiply-adds",
             "peak_source": "measured in this run: best of mad.lo / mad.hi / carry-chain probes "
@@ -417,7 +416,7 @@ def run_ours(a, d: Dist) -> dict | None:
             "unit": "GB/s",
             "frac": round(ntt_gbs / hbm_peak, 4),
             "peak_source": hbm_src,
-            "traffic": NCU_TRAFFIC.get(f"ntt_form{ntt.params()['variant']}_2^24"),
+            "traffic": NCU_TRAFFIC.get(f"ntt_form{ntt.params()['variant']}_2^{a.log_ntt}"),
             "algorithmic": "64 B per element per pass (read + write), beside the passes' twiddle tables",
             "transform_frac_of_hbm": round((ntt_bytes * n_pass / (sum(stn.values()) * 1e-3) / 1e9) / hbm_peak, 4),
             "product_rate": {
