@@ -607,13 +607,14 @@ uint32_t NttPlan::tile_log() const { return variant != 0 ? kTileLogD : kTileLog;
 
 bool NttPlan::set_variant(int v) {
   if (v < 0 || v > 4) return false;
-  if (v <= 1 && !fwd_tw.ptr) {  // the table of w^j on first use of a form that reads it
+  // The inverse's tables come last: where they are there, so are the forward's.
+  if (v <= 1 && !inv_tw.ptr) {  // the table of w^j on first use of a form that reads it
     use(ctx);
     build_twiddles(seeds[0], fwd_tw);
     build_twiddles(seeds[1], inv_tw);
     check_cuda(cudaStreamSynchronize(ctx->setup), "ntt twiddles");
   }
-  if (v == 1 && !fwd_twd.ptr) {  // twiddle limbs on first use of the double-precision form
+  if (v == 1 && !inv_twd.ptr) {  // twiddle limbs on first use of the double-precision form
     const size_t count = (size_t)1 << (log_n - 1);
     use(ctx);
     fwd_twd.alloc(10 * count, "ntt twiddle limbs");
@@ -791,6 +792,8 @@ void NttPlan::prepare_shift(const CosetShift& shift) { fused_for(shift); }
 void NttPlan::enqueue(uint32_t* data, bool inverse, cudaStream_t s, const CosetShift* shift, const Quotient* quot) {
   if (shift && !inverse) fail(ZKG_EINVAL, "a fused coset shift follows an inverse transform");
   if (quot && inverse) fail(ZKG_EINVAL, "a fused quotient follows a forward transform");
+  if (variant >= 2 && stage_tw[1].size() != passes.size())  // neither a new form nor the old one fitted (choose)
+    fail(ZKG_ENOMEM, "the NTT plan has no twiddle tables: its last change of form ran out of device memory");
   if (quot && variant < 2) {  // forms without the fused epilogue: the transform, then the kernel
     enqueue(data, false, s);
     quotient(data, quot->a, quot->b, data, log_n, quot->zinv, s);
