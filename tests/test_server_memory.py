@@ -1,6 +1,7 @@
 """The server's HBM budget holds as many slots as without affine rounds: slots have the rounds' scratch only
 while nothing else needs the bytes."""
 import re
+import threading
 
 import numpy as np
 import pytest
@@ -148,4 +149,35 @@ def test_slots_at_work_give_their_scratch_when_done(gpu, sizes, expected):
     stats = server.stats()
     assert stats["slots"] == 2 + count and stats["slots_evicted"] == 0 and stats["bytes_used"] <= stats["budget"]
     check_requests(server, expected, [(LARGE, 5), (SMALL, 4)])
+    server.close()
+
+
+def reserve_beside(server, log_m, count):
+    """Starts reserve(log_m, count) in a thread and returns it with the bytes taken for the first slot, while
+    that slot is still being made."""
+    before = server.stats()["bytes_used"]
+    thread = threading.Thread(target=server.reserve, args=(log_m, count))
+    thread.start()
+    while True:
+        taken = server.stats()["bytes_used"] - before
+        if taken or not thread.is_alive():
+            return thread, taken
+
+
+def test_a_slot_being_reserved_gives_its_scratch_to_one_asked_for_beside_it(gpu, sizes, expected):
+    server = sizes.server(gpu, 1, 16 << 30)
+    thread, estimate = reserve_beside(server, LARGE, 1)  # with rounds
+    thread.join()
+    server.close()
+    server = sizes.server(gpu, 1, 2 * estimate)
+    small = 0
+    while 2 * estimate - server.stats()["bytes_used"] >= estimate + sizes.small_estimate:
+        small += 1
+        server.reserve(SMALL, small)
+    thread, taken = reserve_beside(server, LARGE, 1)
+    server.reserve(SMALL, small + 1)  # fits once the large slot is there and has given up its rounds
+    thread.join()
+    stats = server.stats()
+    assert taken == estimate and stats["slots"] == small + 2 and stats["bytes_used"] <= stats["budget"]
+    check_requests(server, expected, [(LARGE, 3), (SMALL, 4)])
     server.close()

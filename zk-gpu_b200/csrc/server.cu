@@ -520,7 +520,7 @@ void Server::reserve(uint32_t log_m, uint32_t count) {
         need = estimate_bytes(log_m, rounds);
         if (bytes_used + need <= budget) break;
         const size_t shortage = bytes_used + need - budget;
-        if (held < shortage && building == 0)  // a slot being made may come to hold some
+        if (held < shortage && building == 0 && reserving == 0)  // a slot being made may come to hold some
           fail(ZKG_ENOMEM, "slot of 2^" + std::to_string(log_m) + " does not fit the HBM budget (" +
                                std::to_string(budget - std::min(budget, bytes_used)) + " bytes left, " +
                                std::to_string(need) + " needed)");
@@ -528,6 +528,7 @@ void Server::reserve(uint32_t log_m, uint32_t count) {
         cv.wait(lock);
       }
       bytes_used += need;
+      reserving++;
     }
     std::unique_ptr<ServerSlot> s;
     const double t0 = now_ms();
@@ -536,11 +537,14 @@ void Server::reserve(uint32_t log_m, uint32_t count) {
     } catch (...) {
       std::lock_guard<std::mutex> lock(mu);
       bytes_used -= std::min(bytes_used, need);
+      reserving--;
+      cv.notify_all();
       throw;
     }
     {
       std::lock_guard<std::mutex> lock(mu);
       build_ms += now_ms() - t0;
+      reserving--;
       bytes_used = bytes_used - std::min(bytes_used, need) + s->bytes;
       slots_created++;
       slots.push_back(std::move(s));

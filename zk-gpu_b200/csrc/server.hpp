@@ -72,6 +72,7 @@ struct Server {
   };
   std::deque<Build> builds;
   int building = 0;  // slots under construction (each holds a lane)
+  int reserving = 0;  // slots under construction in reserve()
   // Per size: slots reserved by reserve(), slots under construction. A request whose size has
   // max(2, reserved) slots (built or being built), all busy, waits for one of them instead of
   // having another built: under load a build takes tens to hundreds of ms, longer than the wait.
