@@ -173,7 +173,8 @@ int zkg_msm_windows(const zkg_msm *msm, uint32_t *windows, int *glv);
  * smaller slice to bound the plan's device memory (0 restores the largest; values above it are
  * clamped; re-sizes the scratch, synchronising with queued work). A fixed-base plan runs in one
  * pass (ZKG_EINVAL). zkg_msm_passes reports the slice and the number of passes. The result is
- * the same point for every slice size. */
+ * the same point for every slice size. Where this or another call that re-sizes a plan's scratch returns
+ * ZKG_ENOMEM, the plan has none: its runs return ZKG_ENOMEM too until a size fits. */
 int zkg_msm_set_chunk(zkg_msm *msm, size_t points);
 int zkg_msm_passes(const zkg_msm *msm, size_t *chunk, size_t *passes);
 /* Affine rounds (no reference counterpart): from 2^23 (window, point) entries on (G2 2^22), a plan in its
